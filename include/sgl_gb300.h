@@ -342,7 +342,7 @@ sgl_status sgl_sur_nodes_exact(sgl_ctx* ctx, int n, const int32_t* planes, const
 /* Cosmology tables ------------------------------------------------------------------------------------
  * Replaces the chain's Cosmology (sgl.py:65-640 as pipeline.make_cosmology builds it, pipeline.py:39-79:
  * EH98 transfer, smooth-k sigma(M) window with the top-hat sigma_8 anchor, Ludlow+16 concentrations, the
- * growth ODE, radiation Omega_r = Om / (1 + z_eq)) for n cosmologies at once, one CTA each.  params: n x 9
+ * growth ODE, radiation Omega_r = Om / (1 + z_eq)) for n cosmologies at once.  params: n x 9
  * (h, Om, Ob, s8, ns, zeq, Ok, w0, wa), checked against the reference's domain (SGL_ERR_VALUE).  At the nz
  * ascending redshifts z: E, chi (radial comoving distance, Mpc), DM (transverse), D (growth, D(0) = 1), each
  * n x nz; at the nm masses M (Msun): sigmaM (sigma(M) at z = 0) and dlnsig (d ln sigma / d ln M), n x nm; at
