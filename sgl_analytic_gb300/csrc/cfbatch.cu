@@ -11,14 +11,14 @@
 // of CTAs takes items from a device counter until none is left; each item stages its instance's
 // cells through shared memory (all threads of the CTA work on the same instance) and writes its
 // k-points' ln Phi.  Per-term arithmetic is that of the 1-D sweep: FP64 sincos (SGL_FP64), or the
-// float-float phase with exact reduction and FP32 polynomial sin / cos, Kahan-compensated FP32
-// partial sums folded into FP64 every tile of cells (SGL_MIXED).
+// packed FP32 terms of cfterm.cuh with Kahan sums folded into FP64 every tile of cells (SGL_MIXED).
 //
 // Then per instance Phi = exp(ln Phi) times the trapezoid weights, and the inversion to
 //   dP/dln mu = (1 - kappa) / 2 * (1/pi) sum_n w_n Re[Phi(k_n) e^{-i k_n kappa}],  kappa = 1 - mu^-1/2
 // at the caller's ln mu points: one thread per (instance, ln mu point), the instance's Phi staged
 // in shared memory, the phase rotated step by step and re-seeded exactly every 32 steps (FP32
 // rotation from a float-float phase in mixed precision, FP64 rotation from an FP64 phase in FP64).
+#include "cfterm.cuh"
 #include "kernels.cuh"
 
 namespace sgl {
@@ -43,17 +43,25 @@ struct CfbArgs {
 
 // compensated sum over cells [c0, c1) for one k (thread), cells staged cooperatively
 template <int MODE, int KT>
-__device__ __forceinline__ double2 cfb_cells(const CfbArgs& a, long long c0, long long c1, double k, ff kf,
-                                             float4* s_c, double* s_k, double* s_w) {
+__device__ __forceinline__ double2 cfb_cells(const CfbArgs& a, long long c0, long long c1, double k, const CfWave& kf, float khm,
+                                             float (*s_f)[MODE == SGL_FP64 ? 4 : kCfbTile], double* s_k, double* s_w) {
     double ar = 0.0, ai = 0.0;
     for (long long base = c0; base < c1; base += kCfbTile) {
         const int cnt = (int)((c1 - base) < kCfbTile ? (c1 - base) : kCfbTile);
         __syncthreads();
-        for (int e = threadIdx.x; e < cnt; e += KT) {
+        bool big = false;
+        const int cnt8 = (cnt + kCfGroup - 1) / kCfGroup * kCfGroup;
+        for (int e = threadIdx.x; e < (MODE == SGL_FP64 ? cnt : cnt8); e += KT) {
             if (MODE == SGL_FP64) { s_k[e] = a.kap[base + e]; s_w[e] = a.w[base + e]; }
-            else s_c[e] = make_float4(a.kh[base + e], a.kl[base + e], a.wf[base + e], 0.f);
+            else {
+                const bool in = e < cnt;
+                s_f[0][e] = in ? a.kh[base + e] : 0.f;
+                s_f[1][e] = in ? a.kl[base + e] : 0.f;
+                s_f[2][e] = in ? a.wf[base + e] : 0.f;
+                big |= fabsf(s_f[0][e]) * khm > kCfBigHalfPhase;
+            }
         }
-        __syncthreads();
+        big = __syncthreads_or(big);
         if (MODE == SGL_FP64) {
             for (int e = 0; e < cnt; ++e) {
                 const double ph = k * s_k[e];
@@ -71,33 +79,13 @@ __device__ __forceinline__ double2 cfb_cells(const CfbArgs& a, long long c0, lon
                 ai = fma(s_w[e], smp, ai);
             }
         } else {
-            float far = 0.f, fai = 0.f, car = 0.f, cai = 0.f;
-            for (int e = 0; e < cnt; ++e) {
-                const float4 cv = s_c[e];
-                ff kapf; kapf.hi = cv.x; kapf.lo = cv.y;
-                float r, ph_hi, ph_lo;
-                int qi;
-                halfangle_reduce_ff(kf, kapf, r, qi, ph_hi, ph_lo);
-                float sr, cr;
-                sincos_reduced(r, sr, cr);
-                const bool odd = qi & 1;
-                const float av = odd ? cr : sr;
-                const float cm1 = -2.f * av * av;
-                const float sn = (odd ? -2.f : 2.f) * sr * cr;
-                const float ph = ph_hi + ph_lo;
-                float smp;
-                if (fabsf(ph) < 1e-2f) {
-                    const float p2 = ph * ph;
-                    smp = -ph * p2 * (1.f / 6.f) * (1.f - p2 * (1.f / 20.f) * (1.f - p2 * (1.f / 42.f)));
-                } else {
-                    smp = (sn - ph_hi) - ph_lo;
-                }
-                const float wv = cv.z;
-                float y = fmaf(wv, cm1, -car); float t = far + y; car = (t - far) - y; far = t;
-                y = fmaf(wv, smp, -cai); t = fai + y; cai = (t - fai) - y; fai = t;
-            }
-            ar += (double)far - (double)car;
-            ai += (double)fai - (double)cai;
+            CfSums S;
+            S.clear();
+            if (big) cf_tile<true>(kf, s_f[0], s_f[1], s_f[2], cnt8, S);
+            else cf_tile<false>(kf, s_f[0], s_f[1], s_f[2], cnt8, S);
+            const double2 v = S.value();
+            ar += v.x;
+            ai += v.y;
         }
     }
     return make_double2(ar, ai);
@@ -106,7 +94,7 @@ __device__ __forceinline__ double2 cfb_cells(const CfbArgs& a, long long c0, lon
 template <int MODE, int KT>
 __global__ void __launch_bounds__(KT)
 k_cfb_persistent(CfbArgs a) {
-    __shared__ float4 s_c[MODE == SGL_FP64 ? 1 : kCfbTile];
+    __shared__ __align__(16) float s_f[3][MODE == SGL_FP64 ? 4 : kCfbTile];
     __shared__ double s_k[MODE == SGL_FP64 ? kCfbTile : 1];
     __shared__ double s_w[MODE == SGL_FP64 ? kCfbTile : 1];
     __shared__ double s_K[kCfbMaxStates * kCfbMaxStates];
@@ -122,11 +110,14 @@ k_cfb_persistent(CfbArgs a) {
         const CfbInst I = a.inst[wi.x];
         const int n = wi.y * KT + threadIdx.x;
         const bool live = n < I.nk;
-        const double k = live ? (I.geom ? exp(I.k0 + (double)n * I.dk) : I.k0 + (double)n * I.dk) : 0.0;
-        const ff kf = ff_from_double(k);
+        auto k_at = [&](int j) { return I.geom ? exp(I.k0 + (double)j * I.dk) : I.k0 + (double)j * I.dk; };
+        const double k = live ? k_at(n) : 0.0;
+        const CfWave kf(k);
+        // the item's largest half wave number (k ascends)
+        const float khm = MODE == SGL_FP64 ? 0.f : 0.5f * (float)fmax(fabs(k_at(wi.y * KT)), fabs(k_at(min(I.nk, wi.y * KT + KT) - 1)));
         double2 lp;
         if (I.closure == 0) {
-            const double2 s = cfb_cells<MODE, KT>(a, I.c0, I.c1, k, kf, s_c, s_k, s_w);
+            const double2 s = cfb_cells<MODE, KT>(a, I.c0, I.c1, k, kf, khm, s_f, s_k, s_w);
             lp = make_double2(s.x - 0.5 * I.V * k * k, s.y);
         } else if (MODE == SGL_FP64) {
             // Poisson sum plus the chain: alpha_t = (sum_s alpha_s K_st) e^{z_t}, z_t = D_pt Lambda_p,
@@ -136,7 +127,7 @@ k_cfb_persistent(CfbArgs a) {
             double ar[kCfbMaxStates], ai[kCfbMaxStates];
             double lnsc = 0.0, sr = 0.0, si = 0.0;
             for (int p = I.p0; p < I.p1; ++p) {
-                const double2 L = cfb_cells<MODE, KT>(a, a.plane_cells[p], a.plane_cells[p + 1], k, kf, s_c, s_k, s_w);
+                const double2 L = cfb_cells<MODE, KT>(a, a.plane_cells[p], a.plane_cells[p + 1], k, kf, khm, s_f, s_k, s_w);
                 sr += L.x; si += L.y;
                 const double* D = a.vp_D + (long long)p * S;
                 double br[kCfbMaxStates], bi[kCfbMaxStates];
@@ -197,7 +188,7 @@ k_cfb_persistent(CfbArgs a) {
             float ar[kCfbMaxStates], ai[kCfbMaxStates];
             double lnsc = 0.0, sr = 0.0, si = 0.0;
             for (int p = I.p0; p < I.p1; ++p) {
-                const double2 L = cfb_cells<MODE, KT>(a, a.plane_cells[p], a.plane_cells[p + 1], k, kf, s_c, s_k, s_w);
+                const double2 L = cfb_cells<MODE, KT>(a, a.plane_cells[p], a.plane_cells[p + 1], k, kf, khm, s_f, s_k, s_w);
                 sr += L.x; si += L.y;
                 const double* D = a.vp_D + (long long)p * S;
                 float br[kCfbMaxStates], bi[kCfbMaxStates];
