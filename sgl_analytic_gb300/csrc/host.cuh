@@ -420,9 +420,90 @@ inline void resolve_stats(sgl_ctx* c) {
 }
 
 // ------------------------------------------------------------------ GEMM dispatch
+// device error flag of this context (zeroed on first use)
+inline int* dev_err_flag(sgl_ctx* ctx) {
+    if (!ctx->dev_err) {
+        ctx->dev_err = (int*)ctx->arena.get("dev_err", sizeof(int));
+        if (ctx->dev_err) cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), ctx->stream);
+    }
+    return ctx->dev_err;
+}
+
+// FP64 GEMMs of at least this many FLOP in all run sliced on the tensor cores (oz_gemm.cu); below, its four launches and
+// unsplit K cost more than they save (0.12 GFLOP: 0.24 ms sliced, 0.14 ms SIMT; 0.07: 0.11 and 0.07; 6.9: 0.52 and 5.8)
+constexpr double kOzMinFlops = 4e8;
+constexpr long long kOzBatchBytes = 1LL << 30;    // packed digits of one batch
+
+// The GEMMs of `d` in batches whose digits take at most kOzBatchBytes (a larger problem in slices of rows).  *ran = false
+// (nothing launched) when one does not fit that way or the scratch cannot be had: the caller takes the SIMT kernel.
+inline sgl_status run_oz_gemms(sgl_ctx* ctx, const std::vector<GemmDesc<double>>& d, const std::string& tag, bool* ran) {
+    *ran = false;
+    struct Batch { std::vector<OzGemmDesc> g; long long bytes = 0; };
+    std::vector<Batch> batches;
+    auto digits = [](long long rows, int K) { return (rows + 127) / 128 * 128 * ((K + 31) / 32) * 64 * 7; };
+    double fl = 0.0;
+    for (const auto& g : d) {
+        const long long bb = digits(g.N, g.K), room = kOzBatchBytes - bb, per = digits(128, g.K);
+        if (room < per) return SGL_OK;
+        const int step = (int)std::min<long long>(room / per * 128, 1 << 30);
+        for (int i0 = 0; i0 < g.M; i0 += step) {
+            OzGemmDesc o{};
+            o.M = std::min(step, g.M - i0); o.N = g.N; o.K = g.K;
+            o.A = g.A + (long long)i0 * g.a_rs; o.a_rs = g.a_rs; o.a_cs = g.a_cs;
+            o.B = g.B; o.b_rs = g.b_rs; o.b_cs = g.b_cs;
+            o.C = g.C + (long long)i0 * g.ldc; o.ldc = g.ldc;
+            o.alpha = g.alpha; o.beta = g.beta;
+            const long long need = digits(o.M, o.K) + bb;
+            if (batches.empty() || batches.back().bytes + need > kOzBatchBytes) batches.emplace_back();
+            batches.back().g.push_back(o);
+            batches.back().bytes += need;
+        }
+        fl += 2.0 * g.M * (double)g.N * g.K;
+    }
+    // the xi term may run beside the separable part, on the other stream: buffers of its own
+    const std::string side = tag == "xi" ? "_xi" : "";
+    std::vector<std::vector<OzPackDesc>> packs(batches.size());
+    std::vector<OzPlan> plans(batches.size());
+    size_t nd = 0, scales = 0;
+    long long bytes = 0;
+    for (size_t i = 0; i < batches.size(); ++i) {
+        packs[i].resize(3 * batches[i].g.size());
+        oz_gemm_plan(batches[i].g.data(), (int)batches[i].g.size(), packs[i].data(), &plans[i]);
+        nd += batches[i].g.size();
+        bytes = std::max(bytes, plans[i].bytes);
+        scales = std::max(scales, (size_t)plans[i].scales);
+        if (plans[i].quads / 256 >= (1LL << 31) || plans[i].scale_ctas >= (1LL << 31) || plans[i].k_ctas >= (1LL << 31)) return SGL_OK;
+    }
+    OzGemmDesc* dd = dbuf<OzGemmDesc>(ctx, "oz_desc_" + tag, nd);
+    OzPackDesc* dp = dbuf<OzPackDesc>(ctx, "oz_pack_" + tag, 3 * nd);
+    int* sc = dbuf<int>(ctx, "oz_scale" + side, scales);
+    unsigned char* packed = dbuf<unsigned char>(ctx, "oz_packed" + side, (size_t)bytes);
+    int* err = dev_err_flag(ctx);
+    if (!dd || !dp || !sc || !packed || !err) { cudaGetLastError(); return SGL_OK; }
+    *ran = true;
+    Timed t(ctx, "gemm_oz_" + tag, fl, 0.0);
+    size_t at = 0;
+    for (size_t i = 0; i < batches.size(); ++i) {
+        const size_t n = batches[i].g.size();
+        CKS(upload(ctx, dd + at, batches[i].g.data(), n));
+        CKS(upload(ctx, dp + 3 * at, packs[i].data(), 3 * n));
+        launch_oz_gemm(dd + at, (int)n, dp + 3 * at, plans[i], packed, sc, err, ctx->stream);
+        CKLAUNCH();
+        at += n;
+    }
+    return SGL_OK;
+}
+
 template <typename T>
-inline sgl_status run_gemms(sgl_ctx* ctx, std::vector<GemmDesc<T>>& d, const std::string& tag) {
+inline sgl_status run_gemms(sgl_ctx* ctx, std::vector<GemmDesc<T>>& d, const std::string& tag, bool fma_only = false) {
     if (d.empty()) return SGL_OK;
+    if constexpr (sizeof(T) == 8) if (!fma_only) {
+        double fl = 0.0;
+        for (auto& g : d) fl += 2.0 * g.M * (double)g.N * g.K;
+        bool ran = false;
+        if (fl >= kOzMinFlops) CKS(run_oz_gemms(ctx, d, tag, &ran));
+        if (ran) return SGL_OK;
+    }
     int tiles = gemm_plan(d.data(), (int)d.size());
     // FP64 problems too small for one wave of 64 x 64 tiles run on 16 x 16 tiles
     const bool small = sizeof(T) == 8 && tiles < kNumSMs;
@@ -441,15 +522,6 @@ inline sgl_status run_gemms(sgl_ctx* ctx, std::vector<GemmDesc<T>>& d, const std
     }
     CKLAUNCH();
     return SGL_OK;
-}
-
-// device error flag of this context (zeroed on first use)
-inline int* dev_err_flag(sgl_ctx* ctx) {
-    if (!ctx->dev_err) {
-        ctx->dev_err = (int*)ctx->arena.get("dev_err", sizeof(int));
-        if (ctx->dev_err) cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), ctx->stream);
-    }
-    return ctx->dev_err;
 }
 
 // reads (and clears) the flag; call after the stream has work queued that may raise it
@@ -510,6 +582,10 @@ GemmDesc<T> gd(int M, int N, int K, const void* A, long long ars, long long acs,
 // then a fixed-order sum (deterministic).  SIMT kernels (FP64, and FP32 where chosen below).
 template <typename T>
 inline sgl_status gemm_splitk_simt(sgl_ctx* ctx, GemmDesc<T> g, const std::string& tag, int min_split = 1) {
+    if (sizeof(T) == 8 && 2.0 * g.M * (double)g.N * g.K >= kOzMinFlops) {      // needs no K slices
+        std::vector<GemmDesc<T>> v{g};
+        return run_gemms(ctx, v, tag);
+    }
     GemmDesc<T> tmp = g;
     const int tiles = gemm_plan(&tmp, 1);
     int split = 1;

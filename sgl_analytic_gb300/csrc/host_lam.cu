@@ -422,12 +422,20 @@ sgl_status xi_eval(sgl_ctx* ctx, int precision, const double* d_kk, const double
         }
         CKLAUNCH();
     } else if (precision == SGL_FP64) {
-        std::vector<GemmDesc<double>> v;
+        // The leading row of an m = 0 group has G = sum_p E T - sum rows, a difference of sums of up to 2e4 that cancel
+        // at small k: its rounding is the rounding of the whole term (the next row's counts 1e-3 of it).  That row stays
+        // on the FP64 FMA chain that stored PDFs were made with; on the sliced GEMM the skewness of the z_s = 1 PDF
+        // moves by up to 8e-10 (the chain's own rounding error), with this row kept by less than 1e-10.
+        std::vector<GemmDesc<double>> v, lead;
         for (int g = 0; g < X.n_groups; ++g) {
-            const int N = X.r[g] * nkg;
-            v.push_back(gd<double>(2 * nk, N, X.nP[g], (const double*)E + E_off[g], X.nP[g], 1,
-                                   (const double*)T + T_off[g], N, 1, (double*)G + G_off[g], N));
+            const int N = X.r[g] * nkg, N0 = X.m[g] == 0 ? nkg : 0;
+            const double* Eg = (const double*)E + E_off[g];
+            const double* Tg = (const double*)T + T_off[g];
+            double* Gg = (double*)G + G_off[g];
+            if (N0 > 0) lead.push_back(gd<double>(2 * nk, N0, X.nP[g], Eg, X.nP[g], 1, Tg, N, 1, Gg, N));
+            if (N > N0) v.push_back(gd<double>(2 * nk, N - N0, X.nP[g], Eg, X.nP[g], 1, Tg + N0, N, 1, Gg + N0, N));
         }
+        CKS(run_gemms(ctx, lead, "xi_lead", true));
         CKS(run_gemms(ctx, v, "xi"));
     } else {
         // tensor cores, transposed so that the 2 nk rows of E fit one tile width:

@@ -207,6 +207,27 @@ int tc_drain_bn();
 void launch_tc_gemm(int parts, const TcGemmDesc* d_descs, int nprob, int tiles, const TcPackDesc* d_pack,
                     long long quads, float* packed, int* err, cudaStream_t st);
 
+// ---- FP64 GEMM by exact slicing on the tensor cores (oz_gemm.cu)
+struct OzGemmDesc {
+    int M, N, K;
+    const double* A; long long a_rs, a_cs;  // A(i,k) = A[i*a_rs + k*a_cs]
+    const double* B; long long b_rs, b_cs;  // B(k,j) = B[k*b_rs + j*b_cs]
+    double* C; long long ldc;               // C(i,j) = alpha sum_k A B + beta C(i,j) at C[i*ldc + j]
+    double alpha, beta;
+    // filled by oz_gemm_plan
+    int tile_begin, tiles_n, Mpad, Npad, sa_off, sb_off;
+    long long a_off, b_off;                 // packed digits (bytes into the packed buffer)
+};
+struct OzPackDesc {                         // one operand to slice: X(r, k) = X[r*x_rs + k*x_cs]
+    const double* X; long long x_rs, x_cs;
+    int R, K, Rpad, nkb, scale_off, k_off, k_sign;
+    long long out_off, quad_begin, scale_begin;
+};
+struct OzPlan { int tiles, scales; long long bytes, quads, scale_ctas, k_ctas; };
+void oz_gemm_plan(OzGemmDesc* d, int n, OzPackDesc* pk, OzPlan* out);
+void launch_oz_gemm(const OzGemmDesc* d_descs, int n, const OzPackDesc* d_pack, const OzPlan& P, unsigned char* packed,
+                    int* scale, int* err, cudaStream_t st);
+
 // gauss stage A of the mixed path written as the packed (2-part TF32) A operand of the xi GEMM
 bool xi_stageA_pack_fits(int r_max, int nkg);
 void launch_xi_stageA_pack(const XiDevice& x, const long long* d_p_prefix, const float* J, int nkg,
