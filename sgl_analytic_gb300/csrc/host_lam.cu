@@ -667,7 +667,19 @@ sgl_status lambda_eval(sgl_ctx* ctx, int precision, const double* h_kk, int nk, 
         {
             Timed t(ctx, precision == SGL_FP64 ? "sep_sweep_f64" : "sep_sweep_mixed", (double)nk * ctx->sep.n_cells,
                     (double)ctx->sep.n_cols * ld * es);
-            launch_sep_sweep(precision, d_kk, nk, ctx->sepd, Tt, d_Ap, d_A1, st);
+            // FP64 rows k_n = k_0 + n dk >= 0 up to their rounding (the inversion's linspace) take the uniform sweep;
+            // two table entries of 16 B per row and cell pay from about one warp of rows on
+            double dk = 0.0;
+            double2* tab = nullptr;
+            if (precision == SGL_FP64 && nk >= 64 && ctx->sepd.n_cells < (1 << 26) && h_kk[0] >= 0.0) {
+                dk = (h_kk[nk - 1] - h_kk[0]) / (nk - 1);
+                bool uniform = dk > 0.0;
+                for (int i = 0; i < nk && uniform; ++i)
+                    uniform = std::fabs(h_kk[i] - (h_kk[0] + i * dk)) <= 1e-14 * h_kk[nk - 1];
+                if (uniform) tab = dbuf<double2>(ctx, "sep_half_angles", 32 * (size_t)ctx->sepd.n_cells);
+                if (!tab) cudaGetLastError();
+            }
+            launch_sep_sweep(precision, d_kk, nk, ctx->sepd, Tt, d_Ap, d_A1, st, dk, tab);
         }
         CKLAUNCH();
         if (precision == SGL_FP64) CKS(sep_gemms<double>(ctx, precision, h_kg, d_kg, nk, nkg, Tt, Gout));

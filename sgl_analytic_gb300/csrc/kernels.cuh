@@ -26,8 +26,9 @@ int psi1_direct_chunks(int64_t nc);
 void launch_psi1_direct(const double* kk, int nk, const double* kg, int nkg, const double* k0,
                         const double* g0, const double* w0, int64_t nc, double* re, double* im,
                         double2* part, cudaStream_t st, int precision = SGL_FP64);
+// tab (FP64, rows uniform with step dk; n_cells x 32): half-angle table of the uniform sweep; nullptr: rows of any spacing
 void launch_sep_sweep(int precision, const double* kk, int nk, const SepDevice& s, void* Tt,
-                      double2* A_part, double2* A1, cudaStream_t st);
+                      double2* A_part, double2* A1, cudaStream_t st, double dk = 0.0, double2* tab = nullptr);
 void launch_j0m1_table(int precision, const double* nodes, int nn, const double* x, int nx, void* B,
                        cudaStream_t st);
 void launch_cheb_matrix(int precision, double K, int N, const double* tpts, const double* x, int nx, void* L,

@@ -18,7 +18,7 @@
 // are 28 / 4096 of a clock per FP64 FMA.  Bound by the MMAs' operand reads from L2: a 128 x 64 tile moves 84 KB per
 // 32 k, 900 tensor clocks per 16.  Measured (FP64 SIMT before -> with slicing): sep1 3366 x 580 x 6384 25.2 -> 1.10 ms,
 // Hankel 3366 x 796 x 2687 11.0 -> 0.64, kappa 2400 x 798 x 3366 13.8 -> 0.63, sep2 3366 x 2687 x 446 6.8 -> 0.56, the xi
-// groups (67 GFLOP, K about 300) 70.4 -> 7.7; rms error on such data 6e-17 .. 5e-16 against 6e-16 .. 3e-15.
+// groups (67 GFLOP, K about 300) 70.4 -> 6.5; rms error on such data 6e-17 .. 5e-16 against 6e-16 .. 3e-15.
 //
 // Layout: operands packed by k_oz_pack as [k block of 32][digit][row][64 B] in the canonical K-major core-matrix
 // layout (as tc_gemm.cu), so that one bulk copy moves a tile's digit.  One CTA per 128 x 64 tile: the seven
@@ -267,6 +267,7 @@ k_oz_gemm(const OzGemmDesc* __restrict__ descs, int nprob, const unsigned char* 
         const int gi = i0 + (warp & 3) * 32 + lane, jb = j0 + (warp >> 2) * kCols;
         if (ok && gi < d.M) {
             const int ea = scale[d.sa_off + gi];
+            const bool scaled = d.alpha != 1.0;
             double* C = d.C + (long long)gi * d.ldc;
 #pragma unroll
             for (int c = 0; c < kCols; ++c) {
@@ -274,10 +275,16 @@ k_oz_gemm(const OzGemmDesc* __restrict__ descs, int nprob, const unsigned char* 
                 if (gj < d.N) {
                     const int eb = scale[d.sb_off + gj];
                     // 2^48 of the weights, 2^(e - 1077) of each operand's integers
+                    // (FP64 instructions count here: 8192 outputs at 2 per clock; the scaling is an integer addition)
                     double v = fma((double)hi[c], 16777216.0, (double)lo[c]);
-                    if (v != 0.0) v = scalbn(v, ea + eb - 2 * kOzBias - 2106);
+                    const int sh = ea + eb - 2 * kOzBias - 2106;
+                    const int ex = (__double2hiint(v) >> 20) & 0x7ff;
+                    if (ex != 0) {
+                        if (ex + sh > 0 && ex + sh < 0x7ff) v = __hiloint2double(__double2hiint(v) + (sh << 20), __double2loint(v));
+                        else v = scalbn(v, sh);
+                    }
                     if (ea >= kOzNan || eb >= kOzNan) v = __longlong_as_double(0x7ff8000000000000LL);
-                    v *= d.alpha;
+                    if (scaled) v *= d.alpha;
                     if (d.beta != 0.0) v = fma(d.beta, C[gj], v);
                     C[gj] = v;
                 }

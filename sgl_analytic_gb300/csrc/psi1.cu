@@ -252,7 +252,7 @@ void launch_psi1_direct(const double* kk, int nk, const double* kg, int nkg, con
 constexpr int kSweepRows = 128;
 constexpr int kSweepStage = 64;
 
-// FP64 sweep (the parity path).
+// FP64 sweep of any rows.
 __global__ void __launch_bounds__(kSweepRows, 4)
 k_sep_sweep_f64(const double* __restrict__ kk, int nk, SepDevice sd, double* __restrict__ Tt,
                 double2* __restrict__ A_part) {
@@ -313,6 +313,103 @@ k_sep_sweep_f64(const double* __restrict__ kk, int nk, SepDevice sd, double* __r
     }
     flush(cur);
     if (live) A_part[(long long)blockIdx.y * nk + n] = make_double2(ar, ai);
+}
+
+// FP64 sweep on a uniform grid of rows (the inversion's).  Bound by the FP64 pipe (2 FMA per clock and SM): of the 91
+// operations a pair took, about 55 were its sincos and 16 are the node sums.  Here the half angle is split as
+// x = x_a + x_b + x_e: k_a the first row of the thread's warp (one sincos per cell and warp, staged), k_b the row's
+// offset in the warp, a multiple of the step (sincos from a table of 32 per cell, 41 MB, L2-resident), and x_e the
+// rounding of the grid points, kappa eps / 2, to first order.  All parts have one sign, so sin x keeps its relative
+// accuracy where 1 - cos and sin - ph need it.  32 operations a pair; 1683 rows x 79,574 cells 20.9 -> 9.1 ms (a third
+// of that through the small-phase series' divisions, now products).
+__global__ void __launch_bounds__(256) k_sep_half_angles(const double* __restrict__ kap, int nc, double dk,
+                                                          double2* __restrict__ tab) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nc * 32) return;
+    double s, c;
+    sincos(0.5 * ((e & 31) * dk) * kap[e >> 5], &s, &c);
+    tab[e] = make_double2(s, c);
+}
+
+__global__ void __launch_bounds__(kSweepRows, 4)
+k_sep_sweep_f64_uniform(const double* __restrict__ kk, int nk, double dk, const double2* __restrict__ tab, SepDevice sd,
+                        double* __restrict__ Tt, double2* __restrict__ A_part) {
+    __shared__ __align__(16) double s_wl[kSweepStage][8];
+    __shared__ double2 s_a[kSweepStage][kSweepRows / 32];
+    __shared__ double2 s_kw[kSweepStage];                       // kappa, weight
+    __shared__ int s_grp[kSweepStage];
+    const int n = blockIdx.x * kSweepRows + threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool live = n < nk;
+    const int na = n - lane;                                    // the warp's first row
+    const double k = live ? kk[n] : 0.0;
+    const double eps = live ? 0.5 * ((k - kk[na]) - lane * dk) : 0.0;
+    const int c_begin = sd.chunk_begin[blockIdx.y], c_end = sd.chunk_begin[blockIdx.y + 1];
+    const long long ld = 2LL * nk;
+    double ar = 0.0, ai = 0.0;                                  // sum w sin^2(x), sum w (sin ph - ph)
+    double tr[8], ti[8];                                        // node sums of cos ph and of sin ph / 2
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { tr[j] = 0.0; ti[j] = 0.0; }
+    int cur = -1;
+    auto flush = [&](int g) {
+        if (g >= 0 && live) {
+            const int col0 = sd.gcol0[g], nc = sd.gncol[g];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (j < nc) {
+                    Tt[(long long)(col0 + j) * ld + n] = tr[j];
+                    Tt[(long long)(col0 + j) * ld + nk + n] = 2.0 * ti[j];
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { tr[j] = 0.0; ti[j] = 0.0; }
+    };
+    for (int base = c_begin; base < c_end; base += kSweepStage) {
+        const int cnt = min(kSweepStage, c_end - base);
+        __syncthreads();
+        for (int e = threadIdx.x; e < cnt; e += kSweepRows) {
+            s_kw[e] = make_double2(sd.kap[base + e], sd.w[base + e]);
+            s_grp[e] = sd.grp[base + e];
+        }
+        for (int e = threadIdx.x; e < cnt * 8; e += kSweepRows) s_wl[e >> 3][e & 7] = sd.wl[(long long)base * 8 + e];
+        for (int e = lane; e < cnt; e += 32) {                  // each warp its own first row
+            double s, c;
+            sincos(0.5 * (na < nk ? kk[na] : 0.0) * sd.kap[base + e], &s, &c);
+            s_a[e][warp] = make_double2(s, c);
+        }
+        __syncthreads();
+        if (na >= nk) continue;
+        const double2* tb = tab + (long long)base * 32 + lane;
+        double2 b = tb[0];
+        for (int e = 0; e < cnt; ++e) {
+            const int g = s_grp[e];
+            if (g != cur) { flush(cur); cur = g; }
+            const double2 a = s_a[e][warp], kw = s_kw[e], bc = b;
+            if (e + 1 < cnt) b = tb[(e + 1) * 32];
+            double s = fma(a.x, bc.y, a.y * bc.x), c = fma(a.y, bc.y, -(a.x * bc.x));
+            const double d = eps * kw.x, s0 = s;
+            s = fma(c, d, s);
+            c = fma(-s0, d, c);
+            const double t = s * s, u = s * c, ph = k * kw.x;
+            double smp;
+            if (fabs(ph) < 1e-2) {
+                const double p2 = ph * ph;
+                smp = -ph * p2 * (1.0 / 6.0) * (1.0 - p2 * (1.0 / 20.0) * (1.0 - p2 * (1.0 / 42.0)));
+            } else {
+                smp = fma(2.0, u, -ph);
+            }
+            ar = fma(kw.y, t, ar);
+            ai = fma(kw.y, smp, ai);
+            const double cr = fma(-2.0, t, 1.0);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                tr[j] = fma(s_wl[e][j], cr, tr[j]);
+                ti[j] = fma(s_wl[e][j], u, ti[j]);
+            }
+        }
+    }
+    flush(cur);
+    if (live) A_part[(long long)blockIdx.y * nk + n] = make_double2(-2.0 * ar, ai);
 }
 
 // Mixed sweep: float-float phase, FP32 sin / cos of the reduced half angle, Kahan-compensated
@@ -422,9 +519,12 @@ __global__ void k_reduce_chunks(const double2* __restrict__ A_part, int nchunks,
 }
 
 void launch_sep_sweep(int precision, const double* kk, int nk, const SepDevice& s, void* Tt,
-                      double2* A_part, double2* A1, cudaStream_t st) {
+                      double2* A_part, double2* A1, cudaStream_t st, double dk, double2* tab) {
     dim3 grid(ceil_div(nk, kSweepRows), s.nchunks);
-    if (precision == SGL_FP64)
+    if (precision == SGL_FP64 && tab) {
+        k_sep_half_angles<<<ceil_div(32LL * s.n_cells, 256), 256, 0, st>>>(s.kap, s.n_cells, dk, tab); SGL_COUNT(1);
+        k_sep_sweep_f64_uniform<<<grid, kSweepRows, 0, st>>>(kk, nk, dk, tab, s, (double*)Tt, A_part); SGL_COUNT(1);
+    } else if (precision == SGL_FP64)
         { k_sep_sweep_f64<<<grid, kSweepRows, 0, st>>>(kk, nk, s, (double*)Tt, A_part); SGL_COUNT(1); }
     else
         { k_sep_sweep_mixed<<<grid, kSweepRows, 0, st>>>(kk, nk, s, (float*)Tt, A_part); SGL_COUNT(1); }

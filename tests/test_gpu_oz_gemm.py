@@ -57,3 +57,21 @@ def test_nan_in_phi_is_reported():
     phi[200, 300] = np.nan
     with pytest.raises(RuntimeError):
         Engine(0).invert_phi(phi, g, np.linspace(-0.2, 0.4, 11), precision=SGL_FP64)
+
+
+@pytest.mark.parametrize("nk", [63, 64, 65, 160])
+@pytest.mark.parametrize("spacing", ["uniform", "offset", "geometric"])
+def test_fp64_sweep_rows(nk, spacing):
+    """The FP64 separable sweep on uniform rows (the split half angles from 64 rows on, a last warp partly filled),
+    on uniform rows that do not start at 0 and on rows of no common step, against the dense sum."""
+    from oracle.lam_oracle import psi1_direct
+    from sgl_analytic_gb300 import Lam, Population
+    pop = Population.load(GOLDEN / "pop_zs1_sub.npz")
+    kk = {"uniform": np.linspace(0.0, 900.0, nk), "offset": np.linspace(3.7, 411.3, nk),
+          "geometric": np.geomspace(1e-4, 900.0, nk)}[spacing]
+    kg = np.linspace(0.0, 700.0, 200000 // nk + 1)
+    L = Lam(pop, xi=False)(kk, kg)
+    i, j = np.unique([0, 1, 31, 32, 33, nk - 2, nk - 1]), np.array([0, 1, 500, kg.size - 1])
+    ref = psi1_direct(pop.k0, pop.g0, pop.w0, kk[i], kg[j])
+    d = np.abs(L[np.ix_(i, j)] - ref)
+    assert np.all(d <= np.where(np.abs(ref) > 100, 1e-12 * np.abs(ref), 1e-10)), d.max()
