@@ -203,6 +203,16 @@ sgl_status sgl_sweep_eval(sgl_ctx* ctx, const double* kk, int nk, int precision,
 sgl_status sgl_gemm_bf16(sgl_ctx* ctx, int M, int N, int K, const float* A, int64_t a_rs, int64_t a_cs,
                          const float* B, int64_t b_rs, int64_t b_cs, float* C, int64_t c_rs, int64_t c_cs,
                          float alpha);
+/* sgl_mlp_layer: one layer's forward pass, Zb = X W + bias and A = silu(Zb) (silu = 1) or Zb, X (M x K), W (K x N),
+ * Zb and A (M x N; either may be NULL) row-major FP32; the operands' BF16 rounding and, with split = 1, X's two BF16
+ * parts (hi, lo) are made while packing and the bias and activation in the GEMM's epilogue.  The same numbers as
+ * sgl_gemm_bf16 on [X_hi | X - X_hi] and [W; W] followed by sgl_mlp_bias_act. */
+sgl_status sgl_mlp_layer(sgl_ctx* ctx, int M, int N, int K, const float* X, const float* W, const float* bias, float* Zb,
+                         float* A, int silu, int split);
+/* sgl_mlp_layer_grad: the gradient through one layer, out = (dZ W^T) * silu'(Zb), dZ (M x K), W (N x K: the layer's
+ * weights, inputs x outputs), Zb and out (M x N; Zb NULL = no activation) row-major FP32: sgl_gemm_bf16 and
+ * sgl_mlp_act_grad in one. */
+sgl_status sgl_mlp_layer_grad(sgl_ctx* ctx, int M, int N, int K, const float* dZ, const float* W, const float* Zb, float* out);
 sgl_status sgl_mlp_bias_act(sgl_ctx* ctx, int M, int N, const float* Z, const float* bias, float* Zb,
                             float* A, int silu);
 sgl_status sgl_mlp_act_grad(sgl_ctx* ctx, int M, int N, const float* dA, const float* Zb, float* dZ);

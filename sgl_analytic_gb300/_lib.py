@@ -22,7 +22,7 @@ EXPORTS = ("sgl_abi_version", "sgl_ctx_create", "sgl_ctx_destroy", "sgl_last_err
            "sgl_ctx_profile", "sgl_stats_json", "sgl_lam_set_cells",
            "sgl_lam_set_xi", "sgl_lam_sigma", "sgl_lnphi", "sgl_xi_term", "sgl_sweep_set_cells", "sgl_sweep_eval", "sgl_measure_peak",
            "sgl_vp_set", "sgl_vp_build", "sgl_vp_lnR", "sgl_invert_opts_default", "sgl_pdf",
-           "sgl_gemm_bf16", "sgl_mlp_bias_act", "sgl_mlp_act_grad", "sgl_mlp_col_sum", "sgl_mlp_mse", "sgl_mlp_adamw",
+           "sgl_gemm_bf16", "sgl_mlp_layer", "sgl_mlp_layer_grad", "sgl_mlp_bias_act", "sgl_mlp_act_grad", "sgl_mlp_col_sum", "sgl_mlp_mse", "sgl_mlp_adamw",
            "sgl_mlp_infer",
            "sgl_plan_grid", "sgl_invert", "sgl_batch_create", "sgl_batch_destroy", "sgl_batch_slots",
            "sgl_batch_slot", "sgl_batch_pdf", "sgl_cfb_set", "sgl_cfb_tune", "sgl_cfb_lnphi", "sgl_cfb_pdf",
@@ -136,6 +136,10 @@ def lib():
             getattr(L, name).restype = C.c_int
         i64, f32 = C.c_int64, C.c_float
         L.sgl_gemm_bf16.argtypes = [vp, C.c_int, C.c_int, C.c_int, vp, i64, i64, vp, i64, i64, vp, i64, i64, f32]
+        L.sgl_mlp_layer.argtypes = [vp, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp, C.c_int, C.c_int]
+        L.sgl_mlp_layer_grad.argtypes = [vp, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp]
+        L.sgl_mlp_layer_grad.restype = C.c_int
+        L.sgl_mlp_layer.restype = C.c_int
         L.sgl_mlp_bias_act.argtypes = [vp, C.c_int, C.c_int, vp, vp, vp, vp, C.c_int]
         L.sgl_mlp_act_grad.argtypes = [vp, C.c_int, C.c_int, vp, vp, vp]
         L.sgl_mlp_col_sum.argtypes = [vp, C.c_int, C.c_int, vp, vp]

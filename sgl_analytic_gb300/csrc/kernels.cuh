@@ -187,6 +187,11 @@ struct TcGemmDesc {
     const float* B; long long b_rs, b_cs;   // B(k,j) = B[k*b_rs + j*b_cs]
     float* C; long long c_rs, c_cs;         // C(i,j) = alpha * sum_k A(i,k) B(k,j) at C[i*c_rs + j*c_cs]
     float alpha;
+    // BF16 mode: split = 1 takes A's FP32 elements as two BF16 parts, [hi | lo] against [B; B] (K counts both, 2 K'
+    // with K' columns of A and rows of B); bias not NULL adds bias[j] and, with act, stores C = z and act = silu(z)
+    // (silu = 1) or z, either output NULL when not wanted
+    int split; const float* bias; float* act; int silu;
+    const float* dact;                      // not NULL: C = alpha sum A B times silu'(dact), dact laid out as C
     // filled by tc_gemm_plan
     int tile_begin, tiles_n, bn, Mpad, Npad;
     long long a_off, b_off;                 // packed operands (floats into the packed buffer)
@@ -194,6 +199,7 @@ struct TcGemmDesc {
 struct TcPackDesc {                         // one operand to pack: X(r, k) = X[r*x_rs + k*x_cs]
     const float* X; long long x_rs, x_cs;
     int R, K, Rpad, nkb;
+    int fold, part;                         // fold = K' > 0: k >= K' reads column k - K' (part: its low part; hi before)
     long long out_off, quad_begin;
 };
 // fills tiles / packing descriptors (pk: 2 n entries) for operands split into `parts` (2 or 3)
@@ -244,7 +250,8 @@ void launch_mlp_fused(int n, const float* X, const float* const* W_dev, const fl
                       float* small, const float** ptrs, float* Y, int* err, int ctas, cudaStream_t st);
 void launch_bias_act(int M, int N, const float* Z, const float* bias, float* Zb, float* A, int silu, cudaStream_t st);
 void launch_act_grad(int M, int N, const float* dA, const float* Zb, float* dZ, cudaStream_t st);
-void launch_col_sum(int M, int N, const float* X, float* out, cudaStream_t st);
+long long col_sum_parts(int M, int N);   // doubles of scratch
+void launch_col_sum(int M, int N, const float* X, double* part, float* out, cudaStream_t st);
 int mse_blocks(long long n);
 void launch_mse(long long n, const float* pred, const float* tgt, float* dpred, double* part, cudaStream_t st);
 void launch_adamw(long long n, float* w, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,

@@ -25,12 +25,29 @@ __global__ void k_act_grad(int M, int N, const float* __restrict__ dA, const flo
     dZ[e] = dA[e] * sg * (1.f + z * (1.f - sg));
 }
 
-// out[j] = sum_i X[i, j]: one CTA per column, FP64 tree
-__global__ void __launch_bounds__(256) k_col_sum(int M, int N, const float* __restrict__ X, float* __restrict__ out) {
+// out[j] = sum_i X[i, j] in FP64: a CTA per (128 columns, 64 rows) adds its rows column by column (coalesced), a second
+// pass adds the CTAs' sums in order.  One CTA per column, 4-byte reads N apart, took 45 us for 16384 x 256; this, 26.
+constexpr int kColRows = 64;
+__global__ void __launch_bounds__(128) k_col_part(int M, int N, int rows, const float* __restrict__ X, double* __restrict__ part) {
+    const int j = blockIdx.x * 128 + threadIdx.x;
+    if (j >= N) return;
+    const int i0 = min((long long)M, (long long)blockIdx.y * rows), i1 = min((long long)M, (long long)i0 + rows);
+    double a0 = 0.0, a1 = 0.0;
+    int i = i0;
+#pragma unroll 4
+    for (; i + 1 < i1; i += 2) {
+        a0 += (double)X[(long long)i * N + j];
+        a1 += (double)X[(long long)(i + 1) * N + j];
+    }
+    if (i < i1) a0 += (double)X[(long long)i * N + j];
+    part[(long long)blockIdx.y * N + j] = a0 + a1;
+}
+
+__global__ void __launch_bounds__(256) k_col_sum(int np, int N, const double* __restrict__ part, float* __restrict__ out) {
     __shared__ double sh[32];
     const int j = blockIdx.x;
     double a = 0.0;
-    for (int i = threadIdx.x; i < M; i += blockDim.x) a += (double)X[(long long)i * N + j];
+    for (int i = threadIdx.x; i < np; i += blockDim.x) a += part[(long long)i * N + j];
     a = block_sum(a, sh);
     if (threadIdx.x == 0) out[j] = (float)a;
 }
@@ -70,8 +87,14 @@ void launch_act_grad(int M, int N, const float* dA, const float* Zb, float* dZ, 
     const long long t = (long long)M * N;
     if (t > 0) { k_act_grad<<<ceil_div(t, 256), 256, 0, st>>>(M, N, dA, Zb, dZ); SGL_COUNT(1); }
 }
-void launch_col_sum(int M, int N, const float* X, float* out, cudaStream_t st) {
-    if (N > 0) { k_col_sum<<<N, 256, 0, st>>>(M, N, X, out); SGL_COUNT(1); }
+int col_sum_rows(int M) { return std::max(kColRows, ceil_div(M, 65535)); }      // rows per CTA: grid.y <= 65535
+long long col_sum_parts(int M, int N) { return (long long)std::max(1, ceil_div(M, col_sum_rows(M))) * N; }
+void launch_col_sum(int M, int N, const float* X, double* part, float* out, cudaStream_t st) {
+    if (N <= 0) return;
+    const int rows = col_sum_rows(M), np = ceil_div(M, rows);
+    if (np > 0) { k_col_part<<<dim3(ceil_div(N, 128), np), 128, 0, st>>>(M, N, rows, X, part); SGL_COUNT(1); }
+    k_col_sum<<<N, 256, 0, st>>>(np, N, part, out);
+    SGL_COUNT(1);
 }
 int mse_blocks(long long n) { return (int)std::min<long long>(1024, std::max<long long>(1, ceil_div(n, 256))); }
 void launch_mse(long long n, const float* pred, const float* tgt, float* dpred, double* part, cudaStream_t st) {

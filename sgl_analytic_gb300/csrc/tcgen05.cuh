@@ -12,7 +12,7 @@ namespace sgl {
 constexpr int kTcBM = 128;                 // tile rows = TMEM lanes
 constexpr int kTcBNmax = 256;              // tile columns = TMEM columns allocated
 constexpr int kTcBK = 16;                  // K per stage: two MMA k-steps of 8 (TF32)
-constexpr int kTcThreads = 128;
+constexpr int kTcThreads = 256;
 constexpr int kTcLBO = 128;                // bytes between core matrices along K
 constexpr int kTcSBO = 512;                // bytes between 8-row groups
 constexpr int kTcAbytes = kTcBM * kTcBK * 4;          // 8 KB per TF32 part

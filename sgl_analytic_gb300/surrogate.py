@@ -123,26 +123,19 @@ class MLP:
         """X: (n, 8) float32 device tensor -> (n, 2); keep=True stores activations for backward."""
         torch, e = self.torch, self.eng
         n = X.shape[0]
-        acts, pre = [X], []
         with torch.cuda.stream(self.stream):
-            A = X
+            A = X.contiguous()
+            acts, pre = [A], []
             for l, (W, b) in enumerate(zip(self.W, self.b)):
                 a, c = W.shape
-                Z = torch.empty((n, c), device=self.dev)
-                if self.split:
-                    # the layer's input as two BF16 parts [A_hi | A_lo] against [W; W]: the product of the
-                    # FP32 input (to 2^-17) with the BF16 weights, FP32 accumulation
-                    Ah = A.to(torch.bfloat16).to(torch.float32)
-                    A2 = torch.cat([Ah, A - Ah], 1)
-                    W2 = torch.cat([W, W], 0)
-                    self._gemm(n, c, 2 * a, A2, 2 * a, 1, W2, c, 1, Z, c, 1)
-                else:
-                    self._gemm(n, c, a, A, a, 1, W, c, 1, Z, c, 1)
-                Zb = torch.empty_like(Z) if keep else Z
-                out = torch.empty_like(Z)
+                # the layer's input as two BF16 parts [A_hi | A_lo] against [W; W] (split): the product of the
+                # FP32 input (to 2^-17) with the BF16 weights, FP32 accumulation
+                Zb = torch.empty((n, c), device=self.dev) if keep else None
+                out = torch.empty((n, c), device=self.dev)
                 last = l == len(self.W) - 1
-                e._check(e._L.sgl_mlp_bias_act(e._h, n, c, Z.data_ptr(), b.data_ptr(), Zb.data_ptr(), out.data_ptr(),
-                                               0 if last else 1), "sgl_mlp_bias_act")
+                e._check(e._L.sgl_mlp_layer(e._h, n, c, a, A.data_ptr(), W.data_ptr(), b.data_ptr(),
+                                            Zb.data_ptr() if keep else None, out.data_ptr(), 0 if last else 1,
+                                            int(self.split)), "sgl_mlp_layer")
                 if keep:
                     pre.append(Zb)
                     acts.append(out)
@@ -157,25 +150,21 @@ class MLP:
         n = dY.shape[0]
         grads = []
         with torch.cuda.stream(self.stream):
-            dA = dY
+            dZ = dY
             for l in range(len(self.W) - 1, -1, -1):
                 W = self.W[l]
                 a, c = W.shape
-                if l == len(self.W) - 1:
-                    dZ = dA
-                else:
-                    dZ = torch.empty_like(dA)
-                    e._check(e._L.sgl_mlp_act_grad(e._h, n, c, dA.data_ptr(), self._pre[l].data_ptr(), dZ.data_ptr()),
-                             "sgl_mlp_act_grad")
                 dW = torch.empty((a, c), device=self.dev)
                 Aprev = self._acts[l]
                 self._gemm(a, c, n, Aprev, 1, a, dZ, c, 1, dW, c, 1)           # A^T dZ
                 db = torch.empty(c, device=self.dev)
                 e._check(e._L.sgl_mlp_col_sum(e._h, n, c, dZ.data_ptr(), db.data_ptr()), "sgl_mlp_col_sum")
                 grads.append((l, dW, db))
-                if l > 0:
-                    dA = torch.empty((n, a), device=self.dev)
-                    self._gemm(n, a, c, dZ, c, 1, W, 1, c, dA, a, 1)           # dZ W^T
+                if l > 0:                                                      # (dZ W^T) silu'(pre-activation)
+                    dprev = torch.empty((n, a), device=self.dev)
+                    e._check(e._L.sgl_mlp_layer_grad(e._h, n, a, c, dZ.data_ptr(), W.data_ptr(),
+                                                     self._pre[l - 1].data_ptr(), dprev.data_ptr()), "sgl_mlp_layer_grad")
+                    dZ = dprev
             self.step_count += 1
             for l, dW, db in grads:
                 for w, g, m, v in ((self.W[l], dW, self.mW[l], self.vW[l]), (self.b[l], db, self.mb[l], self.vb[l])):
