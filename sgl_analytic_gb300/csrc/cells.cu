@@ -7,10 +7,9 @@
 //                  w, w kappa, w gamma and the coarse sums of w beta^n per shell, and per object the
 //                  totals (w, w inside the fine lattice, w kappa over |kappa| < the fine grid's top)
 //                  by a segmented warp scan (points of one object are contiguous).
-//   k_cells_xi     one warp per point inside the coarse box: lanes over the k_perp nodes evaluate
-//                  J0, J2, J4 of k_j R (reused while consecutive points share R and shear type) and add
-//                  beta w J_{2m} into the point's coarse-bin row; the exact first moments accumulate in
-//                  registers and leave once per warp.
+//   k_cells_xi     one CTA per object (or 4096 of its points): points inside the coarse box sorted by radius
+//                  and bin, J0, J2, J4 of k_j R once per radius, beta w J_{2m} added into the coarse-bin rows
+//                  once per radius and bin; the exact first moments leave once per CTA.
 //   k_cells_xi_*   the node's compression (xi_end): occupied rows per m, the residual first-moment row,
 //                  the rows scaled by sqrt(c / dchi), their 42 x 42 Gram matrix (two-stage reduction in
 //                  a fixed order) and the projection onto the kept eigenvectors.
@@ -89,24 +88,37 @@ __device__ __forceinline__ double seg_scan(double x, int lane, int lead) {
 }
 
 // J0, J2, J4 of x as the deposit evaluates them: the power series below x = 2 (3 / 6 / 14 terms below
-// 0.02 / 0.3 / 2), above it J0(x), J1(x) and the upward recurrence J_{n+1} = 2n J_n / x - J_{n-1}
+// 0.02 / 0.3 / 2), above it J0(x), J1(x) and the upward recurrence J_{n+1} = 2n J_n / x - J_{n-1}.  The series by
+// Horner's rule with their coefficients (-1)^k / (k! (k + n)!) as constants: 39 FMAs, where a division per factor of
+// every term took some 600 FP64 operations.
+struct BesselSeries { double c[3][14]; };
+constexpr BesselSeries bessel_series() {
+    BesselSeries s{};
+    for (int n = 0; n < 3; ++n) {
+        double f = 1.0;                                   // 1 / (2 n)!
+        for (int q = 2; q <= 2 * n; ++q) f /= q;
+        s.c[n][0] = f;
+        for (int k = 1; k < 14; ++k) { f /= -(double)k * (double)(k + 2 * n); s.c[n][k] = f; }
+    }
+    return s;
+}
+__constant__ BesselSeries kBessel = bessel_series();
+
 __device__ __forceinline__ void bessel_even(double x, bool tang, double& J0, double& J2, double& J4) {
     if (x < 2.0) {
-        const double h = 0.5 * x, h2 = h * h;
-        double t0 = 1.0, s0 = 1.0, t2 = 0.5, s2 = 0.5, t4 = 1.0 / 24.0, s4 = 1.0 / 24.0;
-        const int nt = x < 0.02 ? 3 : (x < 0.3 ? 6 : 14);
-        for (int k = 1; k < nt; ++k) {
-            const double f = (-h2) / k;
-            t0 *= f / k;
-            s0 += t0;
-            t2 *= f / (k + 2);
-            s2 += t2;
-            t4 *= f / (k + 4);
-            s4 += t4;
+        const double h = 0.5 * x, u = h * h;
+        const bool t14 = x >= 0.3, t6 = x >= 0.02;
+        double s0 = 0.0, s2 = 0.0, s4 = 0.0;
+#pragma unroll
+        for (int k = 13; k >= 0; --k) {
+            const bool on = k < 3 || (k < 6 ? t6 : t14);
+            s0 = fma(s0, u, on ? kBessel.c[0][k] : 0.0);
+            s2 = fma(s2, u, on ? kBessel.c[1][k] : 0.0);
+            s4 = fma(s4, u, on ? kBessel.c[2][k] : 0.0);
         }
         J0 = s0;
-        J2 = tang ? s2 * (h * h) : 0.0;
-        J4 = tang ? s4 * (h * h * h * h) : 0.0;
+        J2 = tang ? s2 * u : 0.0;
+        J4 = tang ? s4 * (u * u) : 0.0;
     } else {
         J0 = j0(x);
         if (tang) {
@@ -177,38 +189,56 @@ __global__ void __launch_bounds__(256) k_cells_hist(CellsGeom G, const double* _
 }
 
 // One CTA per work item (a chunk of at most kXiChunk points of one object).  The chunk's points inside
-// the coarse box are sorted in shared memory by (R, coarse bin); each warp takes runs of one radius,
-// evaluates J0, J2, J4 at the 42 k_perp nodes once for it, merges the radius's points per bin (sum of
-// beta w) and adds v J_{2m} into the bin's row; the radius's sums of beta w kappa and beta w gamma feed
-// the exact first moments.  The same grouping as the reference's default deposit (sgl_full.py:1081-1130).
-__global__ void __launch_bounds__(256) k_cells_xi(CellsGeom G, const double* __restrict__ edges,
-                                                  const CellsXiItem* __restrict__ items,
-                                                  const double* __restrict__ K, const double* __restrict__ Gm,
-                                                  const double* __restrict__ W, const double* __restrict__ R,
-                                                  const double* __restrict__ obj_beta,
-                                                  const unsigned char* __restrict__ obj_tang,
-                                                  const double* __restrict__ kp, int nkp, int mm,
-                                                  double* __restrict__ Hx, double* __restrict__ lx,
-                                                  double* __restrict__ Wb) {
-    __shared__ double s_ek[kCellsXiMaxEdges];
-    __shared__ double s_R[kXiChunk];
-    __shared__ int s_c[kXiChunk], s_i[kXiChunk], s_seg[kXiChunk + 1];
-    __shared__ double s_lx[8][2][64];
-    __shared__ int s_nin, s_nseg;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;     // 256 threads
+// the coarse box are sorted in shared memory by (R, coarse bin).  Runs of one radius are taken kXiBatch at a time:
+// first J0, J2, J4 at every k_perp node of the batch go into shared memory, a warp per node with its lanes over the
+// (ascending) radii, so that they stay on one side of the series' and the large-argument branch; then a warp per
+// radius merges the radius's points per bin (sum of beta w) and adds v J_{2m} into the bin's row; the radius's sums
+// of beta w kappa and beta w gamma feed the exact first moments.  The same grouping as the reference's default
+// deposit (sgl_full.py:1081-1130).
+// Bound by the FP64 pipe (Bessel functions) and the L2's FP64 atomics (126 per radius and bin).  A chunk holds a whole
+// emitted object (12 orientations of 260 radii): with chunks of 1024 every radius was evaluated, and its rows added,
+// three times over.  1.8 M points (512 hosts, 128 filaments): 21.0 -> 3.2 ms.
+constexpr int kXiThreads = 512, kXiBatch = 16;
+constexpr int kXiMaxNodes = 64;
+
+struct XiShared {
+    double R[kXiChunk];
+    unsigned key[kXiChunk];                              // coarse bin << 12 | point of the chunk
+    double J[3][kXiBatch][kXiMaxNodes];
+    double ek[kCellsXiMaxEdges];
+    double lx[kXiThreads / 32][2][kXiMaxNodes];
+    unsigned short seg[kXiChunk + 2];
+    int wsum[kXiThreads / 32];
+    int nin, nseg;
+};
+static_assert(kXiChunk <= 4096, "a point's place takes 12 bits of its sort key");
+
+__global__ void __launch_bounds__(kXiThreads) k_cells_xi(CellsGeom G, const double* __restrict__ edges,
+                                                         const CellsXiItem* __restrict__ items,
+                                                         const double* __restrict__ K, const double* __restrict__ Gm,
+                                                         const double* __restrict__ W, const double* __restrict__ R,
+                                                         const double* __restrict__ obj_beta,
+                                                         const unsigned char* __restrict__ obj_tang,
+                                                         const double* __restrict__ kp, int nkp, int mm,
+                                                         double* __restrict__ Hx, double* __restrict__ lx,
+                                                         double* __restrict__ Wb) {
+    extern __shared__ __align__(16) unsigned char xi_sm[];
+    XiShared& S = *reinterpret_cast<XiShared*>(xi_sm);
+    constexpr int kWarps = kXiThreads / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const CellsXiItem it = items[blockIdx.x];
     const int nekc = G.nekc, negc = G.negc, nkc = nekc - 1, ngc = negc - 1;
     const double* ekc_g = edges + G.nekf + G.negf;
-    for (int t = tid; t < nekc + negc; t += blockDim.x) s_ek[t] = ekc_g[t];
-    if (tid == 0) { s_nin = 0; s_nseg = 0; }
+    for (int t = tid; t < nekc + negc; t += kXiThreads) S.ek[t] = ekc_g[t];
+    if (tid == 0) { S.nin = 0; S.nseg = 0; }
     __syncthreads();
-    const double* ekc = s_ek;
-    const double* egc = s_ek + nekc;
+    const double* ekc = S.ek;
+    const double* egc = S.ek + nekc;
     int n2 = 32;
     while (n2 < it.count) n2 <<= 1;
-    for (int t = tid; t < n2; t += blockDim.x) {
+    for (int t = tid; t < n2; t += kXiThreads) {
         double r = CUDART_INF;
-        int c = 0x7fffffff;
+        unsigned key = 0xffffffffu;
         if (t < it.count) {
             const long long i = it.first + t;
             const double k = K[i];
@@ -218,40 +248,39 @@ __global__ void __launch_bounds__(256) k_cells_xi(CellsGeom G, const double* __r
             const int bc = bin_geom(egc, negc, g, G.gc_lo, G.gc_dl);
             if (ac >= 1 && ac <= nkc && bc >= 1 && bc <= ngc) {
                 r = R[i];
-                c = (ac - 1) * ngc + (bc - 1);
-                atomicAdd(&s_nin, 1);
+                key = (unsigned)((ac - 1) * ngc + (bc - 1)) << 12 | (unsigned)t;
+                atomicAdd(&S.nin, 1);
             }
         }
-        s_R[t] = r;
-        s_c[t] = c;
-        s_i[t] = t;
+        S.R[t] = r;
+        S.key[t] = key;
     }
     __syncthreads();
     // bitonic sort of (R, bin) ascending; points outside the box (R = inf) go last
     for (int k = 2; k <= n2; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int t = tid; t < n2; t += blockDim.x) {
-                const int u = t ^ j;
-                if (u > t) {
-                    const bool gt = s_R[t] > s_R[u] || (s_R[t] == s_R[u] && s_c[t] > s_c[u]);
-                    if (gt == ((t & k) == 0)) {
-                        const double r = s_R[t]; s_R[t] = s_R[u]; s_R[u] = r;
-                        const int c = s_c[t]; s_c[t] = s_c[u]; s_c[u] = c;
-                        const int q = s_i[t]; s_i[t] = s_i[u]; s_i[u] = q;
-                    }
+            for (int p = tid; p < n2 / 2; p += kXiThreads) {
+                const int t = ((p & ~(j - 1)) << 1) | (p & (j - 1)), u = t | j;
+                const double rt = S.R[t], ru = S.R[u];
+                const unsigned ct = S.key[t], cu = S.key[u];
+                const bool gt = rt > ru || (rt == ru && ct > cu);
+                if (gt == ((t & k) == 0)) {
+                    S.R[t] = ru; S.R[u] = rt;
+                    S.key[t] = cu; S.key[u] = ct;
                 }
             }
             __syncthreads();
         }
-    const int nin = s_nin;
+    const int nin = S.nin;
     // starts of the runs of one radius (an emitter's cell centres repeat exactly across orientations),
-    // in order: each thread flags 4 consecutive points, a block-wide exclusive scan places the starts
+    // in order: each thread flags kPer consecutive points, a block-wide exclusive scan places the starts
     {
-        constexpr int kPer = kXiChunk / 256;
+        constexpr int kPer = kXiChunk / kXiThreads;
         int f[kPer], cnt = 0;
+#pragma unroll
         for (int q = 0; q < kPer; ++q) {
             const int t = tid * kPer + q;
-            f[q] = t < nin && (t == 0 || s_R[t] != s_R[t - 1]);
+            f[q] = t < nin && (t == 0 || S.R[t] != S.R[t - 1]);
             cnt += f[q];
         }
         int inc = cnt;
@@ -259,77 +288,100 @@ __global__ void __launch_bounds__(256) k_cells_xi(CellsGeom G, const double* __r
             const int v = __shfl_up_sync(0xffffffffu, inc, d);
             if (lane >= d) inc += v;
         }
-        __shared__ int s_wsum[8];
-        if (lane == 31) s_wsum[warp] = inc;
+        if (lane == 31) S.wsum[warp] = inc;
         __syncthreads();
         int base = inc - cnt;
-        for (int w = 0; w < warp; ++w) base += s_wsum[w];
+        for (int w = 0; w < warp; ++w) base += S.wsum[w];
+#pragma unroll
         for (int q = 0; q < kPer; ++q)
-            if (f[q]) s_seg[base++] = tid * kPer + q;
-        if (tid == 255) s_nseg = base;
-        __syncthreads();
-        if (tid == 0) s_seg[s_nseg] = nin;
+            if (f[q]) S.seg[base++] = (unsigned short)(tid * kPer + q);
+        if (tid == kXiThreads - 1) { S.nseg = base; S.seg[base] = (unsigned short)nin; }
         __syncthreads();
     }
-    const int nseg = s_nseg;
+    const int nseg = S.nseg;
     const double beta = obj_beta[it.obj];
     const bool tang = obj_tang[it.obj] != 0;
-    const bool on0 = lane < nkp, on1 = lane + 32 < nkp;
-    const double kp0 = on0 ? kp[lane] : 0.0, kp1 = on1 ? kp[lane + 32] : 0.0;
     const int mrow = (mm + 1) * nkp;
     double a00 = 0.0, a01 = 0.0, a10 = 0.0, a11 = 0.0;
-    for (int sg = warp; sg < nseg; sg += blockDim.x >> 5) {
-        const int p0 = s_seg[sg], p1 = s_seg[sg + 1];
-        const double r = s_R[p0];
-        double J0a = 0.0, J2a = 0.0, J4a = 0.0, J0b = 0.0, J2b = 0.0, J4b = 0.0;
-        if (on0) bessel_even(kp0 * r, tang, J0a, J2a, J4a);
-        if (on1) bessel_even(kp1 * r, tang, J0b, J2b, J4b);
-        double sk = 0.0, sgm = 0.0;
-        int p = p0;
-        while (p < p1) {                   // runs of one bin within the radius: merged, then one row update
-            const int c = s_c[p];
-            double v = 0.0, ws = 0.0;
-            for (; p < p1 && s_c[p] == c; ++p) {
-                const long long i = it.first + s_i[p];
-                const double w = W[i], k = K[i];
-                double g = Gm[i];
-                g = g < G.g_clip ? G.g_clip : g;
-                const double bw = beta * w;
-                v += bw;
-                ws += w;
-                sk += bw * k;
-                sgm += bw * g;
+    for (int b0 = 0; b0 < nseg; b0 += kXiBatch) {
+        const int nb = min(kXiBatch, nseg - b0);
+        __syncthreads();                                  // the previous batch's readers of J are done
+        // two nodes per warp at a time: 16 radii each
+        for (int q = warp; 2 * q < nkp; q += kWarps) {
+            const int j = 2 * q + (lane >> 4), rr = lane & 15;
+            if (j < nkp && rr < nb) {
+                double J0, J2, J4;
+                bessel_even(kp[j] * S.R[S.seg[b0 + rr]], tang, J0, J2, J4);
+                S.J[0][rr][j] = J0;
+                S.J[1][rr][j] = J2;
+                S.J[2][rr][j] = J4;
             }
-            double* row = Hx + (long long)c * mrow;
-            if (on0) atomicAdd(row + lane, v * J0a);
-            if (on1) atomicAdd(row + lane + 32, v * J0b);
-            if (tang && mm >= 1) {
-                if (on0) atomicAdd(row + nkp + lane, v * J2a);
-                if (on1) atomicAdd(row + nkp + lane + 32, v * J2b);
-                if (mm >= 2) {
-                    if (on0) atomicAdd(row + 2 * nkp + lane, v * J4a);
-                    if (on1) atomicAdd(row + 2 * nkp + lane + 32, v * J4b);
-                }
-            }
-            if (Wb && lane == 0) atomicAdd(Wb + c, ws);
         }
-        a00 += sk * J0a;
-        a01 += sk * J0b;
-        if (tang && mm >= 1) {
-            a10 += sgm * J2a;
-            a11 += sgm * J2b;
+        __syncthreads();
+        for (int rr = warp; rr < nb; rr += kWarps) {
+            const int p0 = S.seg[b0 + rr], p1 = S.seg[b0 + rr + 1];
+            const bool on0 = lane < nkp, on1 = lane + 32 < nkp;
+            const double* Ja = S.J[0][rr];
+            const double* Jb = S.J[1][rr];
+            const double* Jc = S.J[2][rr];
+            double sk = 0.0, sgm = 0.0;
+            int p = p0;
+            while (p < p1) {               // runs of one bin within the radius: merged, then one row update
+                const unsigned c = S.key[p] >> 12;
+                // the run's points one per lane (a radius has few), their sums over the warp
+                int e = p;
+                double v = 0.0, ws = 0.0, vk = 0.0, vg = 0.0;
+                while (e < p1) {
+                    const int t = e + lane;
+                    const bool in = t < p1 && (S.key[t] >> 12) == c;
+                    if (in) {
+                        const long long i = it.first + (S.key[t] & 4095u);
+                        const double w = W[i], k = K[i];
+                        double g = Gm[i];
+                        g = g < G.g_clip ? G.g_clip : g;
+                        const double bw = beta * w;
+                        v += bw; ws += w; vk += bw * k; vg += bw * g;
+                    }
+                    const int n = __popc(__ballot_sync(0xffffffffu, in));
+                    e += n;
+                    if (n < 32) break;
+                }
+                p = e;
+                v = warp_sum(v);
+                if (Wb) ws = warp_sum(ws);
+                sk += warp_sum(vk);
+                sgm += warp_sum(vg);
+                double* row = Hx + (long long)c * mrow;
+                if (on0) atomicAdd(row + lane, v * Ja[lane]);
+                if (on1) atomicAdd(row + lane + 32, v * Ja[lane + 32]);
+                if (tang && mm >= 1) {
+                    if (on0) atomicAdd(row + nkp + lane, v * Jb[lane]);
+                    if (on1) atomicAdd(row + nkp + lane + 32, v * Jb[lane + 32]);
+                    if (mm >= 2) {
+                        if (on0) atomicAdd(row + 2 * nkp + lane, v * Jc[lane]);
+                        if (on1) atomicAdd(row + 2 * nkp + lane + 32, v * Jc[lane + 32]);
+                    }
+                }
+                if (Wb && lane == 0) atomicAdd(Wb + c, ws);
+            }
+            if (on0) a00 += sk * Ja[lane];
+            if (on1) a01 += sk * Ja[lane + 32];
+            if (tang && mm >= 1) {
+                if (on0) a10 += sgm * Jb[lane];
+                if (on1) a11 += sgm * Jb[lane + 32];
+            }
         }
     }
-    s_lx[warp][0][lane] = a00;
-    s_lx[warp][0][lane + 32] = a01;
-    s_lx[warp][1][lane] = a10;
-    s_lx[warp][1][lane + 32] = a11;
+    S.lx[warp][0][lane] = a00;
+    S.lx[warp][0][lane + 32] = a01;
+    S.lx[warp][1][lane] = a10;
+    S.lx[warp][1][lane + 32] = a11;
     __syncthreads();
     if (tid < 2 * nkp) {
         const int m = tid / nkp, j = tid % nkp;
         if (m == 0 || mm >= 1) {
             double s = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += s_lx[w][m][j];
+            for (int w = 0; w < kWarps; ++w) s += S.lx[w][m][j];
             if (s != 0.0) atomicAdd(lx + m * nkp + j, s);
         }
     }
@@ -445,7 +497,8 @@ void launch_cells_xi(const CellsGeom& g, const double* edges, const CellsXiItem*
                      cudaStream_t st) {
     if (n_items <= 0) return;
     SGL_COUNT(1);
-    k_cells_xi<<<n_items, 256, 0, st>>>(g, edges, items, K, Gm, W, R, beta, tang, kp, nkp, mm, Hx, lx, Wb);
+    cudaFuncSetAttribute(k_cells_xi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(XiShared));
+    k_cells_xi<<<n_items, kXiThreads, sizeof(XiShared), st>>>(g, edges, items, K, Gm, W, R, beta, tang, kp, nkp, mm, Hx, lx, Wb);
 }
 
 void launch_cells_xi_tail(const double* kp, int nkp, double coef, double Rm, double* lx, cudaStream_t st) {

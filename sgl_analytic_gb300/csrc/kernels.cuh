@@ -335,7 +335,7 @@ int cells_edge_smem_bytes(const CellsGeom& g);
 void launch_cells_hist(const CellsGeom& g, const double* edges, long long n, const double* K, const double* Gm,
                        const double* W, const long long* off, int n_obj, const int* shell, const double* betas,
                        double* H0, double* H0k, double* H0g, double* Hc, double* sums, int n_sm, cudaStream_t st);
-constexpr int kXiChunk = 1024;            // points of one object per xi work item
+constexpr int kXiChunk = 4096;            // points of one object per xi work item
 constexpr int kCellsXiMaxEdges = 1024;    // coarse kappa + gamma edges the xi kernel holds in shared memory
 struct CellsXiItem { long long first; int count, obj; };
 void launch_cells_xi(const CellsGeom& g, const double* edges, const CellsXiItem* items, int n_items,
