@@ -7,7 +7,8 @@
 //          with Lambda_p the plane's compensated sum and U_p a stationary Markov chain on nstate
 //          latent states (weights w, transition K): the one-dimensional form of the positive Cox
 //          closure (pos_closure.py:184-240, 453-491; one group per plane).
-// Work items are (instance, tile of KT k-points), sorted by cost (longest first).  A persistent grid
+// Work items are (instance, tile of KT k-points, part of a gauss instance's cells), sorted by cost (longest
+// first); parts write partial sums that a second kernel adds in order (k_cfb_sum_parts).  A persistent grid
 // of CTAs takes items from a device counter until none is left; each item stages its instance's
 // cells through shared memory (all threads of the CTA work on the same instance) and writes its
 // k-points' ln Phi.  Per-term arithmetic is that of the 1-D sweep: FP64 sincos (SGL_FP64), or the
@@ -16,8 +17,8 @@
 // Then per instance Phi = exp(ln Phi) times the trapezoid weights, and the inversion to
 //   dP/dln mu = (1 - kappa) / 2 * (1/pi) sum_n w_n Re[Phi(k_n) e^{-i k_n kappa}],  kappa = 1 - mu^-1/2
 // at the caller's ln mu points: one thread per (instance, ln mu point), the instance's Phi staged
-// in shared memory, the phase rotated step by step and re-seeded exactly every 32 steps (FP32
-// rotation from a float-float phase in mixed precision, FP64 rotation from an FP64 phase in FP64).
+// in shared memory, blocks of 32 terms by Horner's rule and an exact phase per block (FP32 blocks with a
+// float-float phase in mixed precision, FP64 in FP64).
 #include "cfterm.cuh"
 #include "kernels.cuh"
 
@@ -28,7 +29,7 @@ constexpr int kCfbMaxStates = 8;
 
 struct CfbArgs {
     const CfbInst* inst;
-    const int2* items;                        // (instance, tile)
+    const int4* items;                        // (instance, tile, part, parts)
     int n_items;
     int* counter;
     const long long* plane_cells;
@@ -39,6 +40,8 @@ struct CfbArgs {
     const double* vp_w;                       // [slot][nstate]
     int nstate;
     double2* out;                             // ln Phi per (instance, k)
+    double2* parts;                           // partial sums [part][instance, k] of split instances
+    long long total_k;
 };
 
 // compensated sum over cells [c0, c1) for one k (thread), cells staged cooperatively
@@ -106,7 +109,7 @@ k_cfb_persistent(CfbArgs a) {
         __syncthreads();
         const int it = s_item;
         if (it >= a.n_items) break;
-        const int2 wi = a.items[it];
+        const int4 wi = a.items[it];
         const CfbInst I = a.inst[wi.x];
         const int n = wi.y * KT + threadIdx.x;
         const bool live = n < I.nk;
@@ -117,7 +120,14 @@ k_cfb_persistent(CfbArgs a) {
         const float khm = MODE == SGL_FP64 ? 0.f : 0.5f * (float)fmax(fabs(k_at(wi.y * KT)), fabs(k_at(min(I.nk, wi.y * KT + KT) - 1)));
         double2 lp;
         if (I.closure == 0) {
-            const double2 s = cfb_cells<MODE, KT>(a, I.c0, I.c1, k, kf, khm, s_f, s_k, s_w);
+            // parts are whole tiles of cells
+            const long long per = ((I.c1 - I.c0 + wi.w - 1) / wi.w + kCfbTile - 1) / kCfbTile * kCfbTile;
+            const long long c0 = min(I.c1, I.c0 + wi.z * per);
+            const double2 s = cfb_cells<MODE, KT>(a, c0, min(I.c1, c0 + per), k, kf, khm, s_f, s_k, s_w);
+            if (wi.w > 1) {
+                if (live) a.parts[wi.z * a.total_k + I.k_off + n] = s;
+                continue;
+            }
             lp = make_double2(s.x - 0.5 * I.V * k * k, s.y);
         } else if (MODE == SGL_FP64) {
             // Poisson sum plus the chain: alpha_t = (sum_s alpha_s K_st) e^{z_t}, z_t = D_pt Lambda_p,
@@ -248,18 +258,42 @@ k_cfb_persistent(CfbArgs a) {
     }
 }
 
+__device__ __forceinline__ int cfb_inst_of(const long long* k_offs, int n_inst, long long e) {
+    int lo = 0, hi = n_inst - 1;                      // the instance whose k range holds e
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (k_offs[mid] <= e) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// ln Phi of the split instances: their parts' sums in order, and the clustering variance
+__global__ void k_cfb_sum_parts(const CfbInst* __restrict__ inst, int n_inst, const long long* __restrict__ k_offs,
+                                const int* __restrict__ nparts, const double2* __restrict__ parts, long long total,
+                                double2* __restrict__ out) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    const int i = cfb_inst_of(k_offs, n_inst, e);
+    const int np = nparts[i];
+    if (np <= 1) return;
+    const CfbInst I = inst[i];
+    double sr = 0.0, si = 0.0;
+    for (int p = 0; p < np; ++p) {
+        const double2 v = parts[p * total + e];
+        sr += v.x;
+        si += v.y;
+    }
+    const double x = I.k0 + (double)(e - I.k_off) * I.dk, k = I.geom ? exp(x) : x;
+    out[e] = make_double2(sr - 0.5 * I.V * k * k, si);
+}
+
 // Phi(k_n) w_n / pi (trapezoid weights) per (instance, k), FP64 or FP32 planes
 template <typename T>
 __global__ void k_cfb_phi(const CfbInst* __restrict__ inst, int n_inst, const double2* __restrict__ lnphi,
                           long long total, const long long* __restrict__ k_offs, T* __restrict__ phi) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
-    int lo = 0, hi = n_inst - 1;                      // the instance whose k range holds e
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (k_offs[mid] <= e) lo = mid; else hi = mid - 1;
-    }
-    const CfbInst I = inst[lo];
+    const CfbInst I = inst[cfb_inst_of(k_offs, n_inst, e)];
     const long long n = e - I.k_off;
     const double wgt = (n == 0 || n == I.nk - 1 ? 0.5 : 1.0) * I.dk / M_PI;
     const double2 L = lnphi[e];
@@ -270,7 +304,7 @@ __global__ void k_cfb_phi(const CfbInst* __restrict__ inst, int n_inst, const do
     phi[2 * e + 1] = (T)(m * s);
 }
 
-constexpr int kCfbPdfThreads = 128;
+constexpr int kCfbPdfThreads = 64;            // small CTAs: a few instances x 2048 points fill more SMs
 constexpr int kCfbPdfStage = 1024;
 constexpr int kCfbReseed = 32;
 
@@ -303,23 +337,25 @@ k_cfb_pdf(const CfbInst* __restrict__ inst, const void* __restrict__ phi_v, cons
         }
         __syncthreads();
         if (MODE == SGL_FP64) {
-            // exact FP64 phase every kCfbReseed steps, FP64 rotation by the step in between
+            // blocks of kCfbReseed terms by Horner's rule in z = e^{-i dk kappa} (4 FMAs a term, a rotated phase takes 6),
+            // then one exact FP64 phase per block
             double sd, cd;
             sincos(I.dk * kap, &sd, &cd);
             for (int e0 = 0; e0 < cnt; e0 += kCfbReseed) {
-                double s, c;
+                double s, c, hr = 0.0, hi = 0.0;
                 sincos((double)(base + e0) * I.dk * kap, &s, &c);
-                const int e1 = min(cnt, e0 + kCfbReseed);
-                for (int e = e0; e < e1; ++e) {
-                    acc = fma(s_pd[e].x, c, fma(s_pd[e].y, s, acc));
-                    const double c2 = fma(c, cd, -s * sd), s2 = fma(s, cd, c * sd);
-                    c = c2;
-                    s = s2;
+#pragma unroll 4
+                for (int e = min(cnt, e0 + kCfbReseed) - 1; e >= e0; --e) {
+                    const double2 f = s_pd[e];
+                    const double t = fma(hr, cd, fma(hi, sd, f.x));
+                    hi = fma(hi, cd, fma(-hr, sd, f.y));
+                    hr = t;
                 }
+                acc = fma(hr, c, fma(hi, s, acc));
             }
         } else {
-            // exact phase (float-float n dk kappa, reduced mod pi/2) every kCfbReseed steps, rotation
-            // by the step's exact sin / cos in between; FP32 terms, FP64 sum per block of steps
+            // the same with FP32 blocks; the block's phase (float-float n dk kappa, reduced mod pi/2) exact, the step's
+            // sine and cosine to FP32, FP64 sum over the blocks
             float sd, cd;
             {
                 float r, ph_hi, ph_lo; int q;
@@ -349,25 +385,27 @@ k_cfb_pdf(const CfbInst* __restrict__ inst, const void* __restrict__ phi_v, cons
                     s = 2.f * shs * chs;
                     c = (chs - shs) * (chs + shs);
                 }
-                float fa = 0.f;
-                const int e1 = min(cnt, e0 + kCfbReseed);
-                for (int e = e0; e < e1; ++e) {
-                    fa = fmaf(s_pf[e].x, c, fmaf(s_pf[e].y, s, fa));
-                    const float c2 = c * cd - s * sd, s2 = s * cd + c * sd;
-                    c = c2; s = s2;
+                float hr = 0.f, hi = 0.f;
+#pragma unroll 8
+                for (int e = min(cnt, e0 + kCfbReseed) - 1; e >= e0; --e) {
+                    const float2 f = s_pf[e];
+                    const float t = fmaf(hr, cd, fmaf(hi, sd, f.x));
+                    hi = fmaf(hi, cd, fmaf(-hr, sd, f.y));
+                    hr = t;
                 }
-                acc += (double)fa;
+                acc += (double)fmaf(hr, c, hi * s);
             }
         }
     }
     if (live) P[(long long)i * nm + m] = acc * (1.0 - kap) * 0.5;
 }
 
-void launch_cfb_persistent(int precision, int kt, int ctas, const CfbInst* inst, const int2* items, int n_items,
+void launch_cfb_persistent(int precision, int kt, int ctas, const CfbInst* inst, const int4* items, int n_items,
                            int* counter, const long long* plane_cells, const double* kap, const double* w,
                            const float* kh, const float* kl, const float* wf, const double* vp_D, const double* vp_K,
-                           const double* vp_w, int nstate, double2* out, cudaStream_t st) {
-    CfbArgs a{inst, items, n_items, counter, plane_cells, kap, w, kh, kl, wf, vp_D, vp_K, vp_w, nstate, out};
+                           const double* vp_w, int nstate, double2* out, cudaStream_t st, double2* parts, int n_inst,
+                           const long long* k_offs, const int* nparts, long long total_k) {
+    CfbArgs a{inst, items, n_items, counter, plane_cells, kap, w, kh, kl, wf, vp_D, vp_K, vp_w, nstate, out, parts, total_k};
     cudaMemsetAsync(counter, 0, sizeof(int), st);
 #define SGL_CFB_LAUNCH(M, T) k_cfb_persistent<M, T><<<ctas, T, 0, st>>>(a)
     if (precision == SGL_FP64) {
@@ -377,6 +415,10 @@ void launch_cfb_persistent(int precision, int kt, int ctas, const CfbInst* inst,
     }
 #undef SGL_CFB_LAUNCH
     SGL_COUNT(1);
+    if (parts) {
+        k_cfb_sum_parts<<<ceil_div(total_k, 256), 256, 0, st>>>(inst, n_inst, k_offs, nparts, parts, total_k, out);
+        SGL_COUNT(1);
+    }
 }
 
 void launch_cfb_pdf(int precision, const CfbInst* inst, int n_inst, const double2* lnphi, long long total,
@@ -394,8 +436,9 @@ void launch_cfb_pdf(int precision, const CfbInst* inst, int n_inst, const double
 }
 
 // Cells of planes with a separable template: cell (m, b) of plane p has kap = u[p][m] F[m][b] and
-// w = v[p][m] g[b] (nm x nb cells per plane, plane after plane), in the solver's FP64, float-float
-// and FP32 forms
+// w = v[p][m] g[b] (nm x nb cells per plane, plane after plane), in the form that the solve's precision reads:
+// FP64 (16 B a cell) or float-float and FP32 (12 B)
+template <bool F64>
 __global__ void k_cfb_fill_separable(long long n_cells, int nm, int nb, const double* __restrict__ F,
                                      const double* __restrict__ g, const double* __restrict__ u,
                                      const double* __restrict__ v, double* __restrict__ kap, double* __restrict__ w,
@@ -408,17 +451,23 @@ __global__ void k_cfb_fill_separable(long long n_cells, int nm, int nb, const do
     const int m = r / nb, b = r - m * nb;
     const double k = u[p * nm + m] * F[r];
     const double ww = v[p * nm + m] * g[b];
-    kap[c] = k;
-    w[c] = ww;
-    const ff f = ff_from_double(k);
-    kh[c] = f.hi;
-    kl[c] = f.lo;
-    wf[c] = (float)ww;
+    if (F64) {
+        kap[c] = k;
+        w[c] = ww;
+    } else {
+        const ff f = ff_from_double(k);
+        kh[c] = f.hi;
+        kl[c] = f.lo;
+        wf[c] = (float)ww;
+    }
 }
 
-void launch_cfb_fill_separable(long long n_cells, int nm, int nb, const double* F, const double* g, const double* u,
-                               const double* v, double* kap, double* w, float* kh, float* kl, float* wf, cudaStream_t st) {
-    k_cfb_fill_separable<<<(unsigned)ceil_div(n_cells, 256), 256, 0, st>>>(n_cells, nm, nb, F, g, u, v, kap, w, kh, kl, wf);
+void launch_cfb_fill_separable(int precision, long long n_cells, int nm, int nb, const double* F, const double* g,
+                               const double* u, const double* v, double* kap, double* w, float* kh, float* kl, float* wf,
+                               cudaStream_t st) {
+    const unsigned n = (unsigned)ceil_div(n_cells, 256);
+    if (precision == SGL_FP64) k_cfb_fill_separable<true><<<n, 256, 0, st>>>(n_cells, nm, nb, F, g, u, v, kap, w, kh, kl, wf);
+    else k_cfb_fill_separable<false><<<n, 256, 0, st>>>(n_cells, nm, nb, F, g, u, v, kap, w, kh, kl, wf);
     SGL_COUNT(1);
 }
 

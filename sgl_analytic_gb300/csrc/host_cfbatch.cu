@@ -15,6 +15,8 @@ struct CfbState {
     int n_inst = 0, n_planes = 0, nstate = 0;
     int shape_class = 0;                       // log2 buckets of the largest k grid and the mean cells
     long long n_cells = 0, total_k = 0;
+    int nm = 0, nb = 0;                        // template planes: the cells' forms present on the device
+    bool have[2] = {true, true};               // (filled per precision on first use)
     std::vector<CfbInst> inst;
     std::vector<double> cost;                  // per instance: cells x k (+ chain) work
     std::vector<int> order;                    // instances by cost, longest first
@@ -45,35 +47,122 @@ void cfb_inst_grid(const CfbState* s, int i, long long* k_off, int* nk, double* 
 namespace sglh {
 namespace {
 
-// work items (instance, k tile) for a tile width, instances in `order`
-std::vector<int2> cfb_items(const CfbState& S, int kt, const std::vector<int>& order) {
-    std::vector<int2> items;
+// work items (instance, k tile, part, parts) for a tile width, instances in `order`, split as `nparts` says
+std::vector<int4> cfb_items(const CfbState& S, int kt, const std::vector<int>& order, const std::vector<int>& nparts) {
+    std::vector<int4> items;
     for (int i : order) {
-        const int tiles = (S.inst[(size_t)i].nk + kt - 1) / kt;
-        for (int t = 0; t < tiles; ++t) items.push_back(make_int2(i, t));
+        const int tiles = (S.inst[(size_t)i].nk + kt - 1) / kt, np = nparts.empty() ? 1 : nparts[(size_t)i];
+        for (int t = 0; t < tiles; ++t)
+            for (int q = 0; q < np; ++q) items.push_back(make_int4(i, t, q, np));
     }
     return items;
 }
 
-sgl_status cfb_launch(sgl_ctx* ctx, int precision, int kt, int cps, const std::vector<int2>& items,
-                      const std::string& tag) {
+// The parts of each gauss instance's cells: a batch with few (instance, k tile) pairs (planes solved at 128 nodes each)
+// would leave CTAs idle or one item running alone at the end, so its items are cut into about four per resident
+// CTA, of at least four tiles of 512 cells.  6 x 64 planes of 131072 cells at 128 nodes: solve 10.6 -> 6.0 ms.
+std::vector<int> cfb_nparts(const CfbState& S, int kt, int ctas, int* most) {
+    long long tiles = 0;
+    for (const CfbInst& I : S.inst) tiles += (I.nk + kt - 1) / kt;
+    const long long want = std::min<long long>(64, (4LL * ctas + tiles - 1) / tiles);
+    *most = 1;
+    std::vector<int> np(S.inst.size(), 1);
+    for (size_t i = 0; i < S.inst.size(); ++i)
+        if (S.inst[i].closure == 0)
+            *most = std::max(*most, np[i] = (int)std::max<long long>(1, std::min(want, (S.inst[i].c1 - S.inst[i].c0) / 2048)));
+    return np;
+}
+
+// a prepared solve: work items, grid and the buffers of split instances
+struct CfbRun {
+    int4* items = nullptr;
+    int n_items = 0, ctas = 0, kt = 0;
+    int* counter = nullptr;
+    double2* lnphi = nullptr; double2* parts = nullptr;
+    int* nparts = nullptr;
+};
+
+sgl_status cfb_prepare(sgl_ctx* ctx, int precision, int kt, int cps, const std::vector<int4>* given, const std::string& tag,
+                       CfbRun& R) {
     CfbState& S = *ctx->cfb;
-    DBUF(d_items, int2, "cfb_items_" + tag, std::max<size_t>(1, items.size()));
-    CKS(upload(ctx, d_items, items.data(), items.size()));
-    DBUF(counter, int, "cfb_counter", 1);
-    DBUF(out, double2, "cfb_lnphi", std::max<long long>(1, S.total_k));
+    const int P = precision == SGL_FP64 ? 0 : 1;
     const int res = cfb_resident_ctas(precision, kt);
     if (res < 1) return fail(ctx, SGL_ERR_CUDA, "batched CF kernel: no resident CTA for this tile width");
-    const int ctas = kNumSMs * std::max(1, std::min(cps, res));
-    launch_cfb_persistent(precision, kt, ctas, (const CfbInst*)ctx->arena.find("cfb_inst"), d_items, (int)items.size(),
-                          counter, (const long long*)ctx->arena.find("cfb_pcells"),
+    R.kt = kt;
+    R.ctas = kNumSMs * std::max(1, std::min(cps, res));
+    int most = 1;
+    std::vector<int4> own;
+    std::vector<int> np;
+    if (!given) {
+        np = cfb_nparts(S, kt, R.ctas, &most);
+        own = cfb_items(S, kt, S.order, np);
+        given = &own;
+    }
+    if (given->size() > (size_t)INT32_MAX) return fail(ctx, SGL_ERR_UNSUPPORTED, "batched CF kernel: too many work items");
+    R.n_items = (int)given->size();
+    R.items = dbuf<int4>(ctx, "cfb_items_" + tag, std::max<size_t>(1, given->size()));
+    R.counter = dbuf<int>(ctx, "cfb_counter", 1);
+    R.lnphi = dbuf<double2>(ctx, "cfb_lnphi", (size_t)std::max<long long>(1, S.total_k));
+    if (!R.items || !R.counter || !R.lnphi) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (batched CF solve)");
+    CKS(upload(ctx, R.items, given->data(), given->size()));
+    if (most > 1) {
+        R.parts = dbuf<double2>(ctx, "cfb_parts_" + tag, (size_t)most * S.total_k);
+        R.nparts = dbuf<int>(ctx, "cfb_nparts_" + tag, np.size());
+        if (!R.parts || !R.nparts) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (batched CF solve)");
+        CKS(upload(ctx, R.nparts, np.data(), np.size()));
+    }
+    if (!S.have[P]) {
+        // template planes: the cells in this precision's form
+        double* kap = nullptr; double* w = nullptr;
+        float* kh = nullptr; float* kl = nullptr; float* wf = nullptr;
+        if (P == 0) {
+            kap = dbuf<double>(ctx, "cfb_kap", (size_t)S.n_cells);
+            w = dbuf<double>(ctx, "cfb_w", (size_t)S.n_cells);
+        } else {
+            kh = dbuf<float>(ctx, "cfb_kh", (size_t)S.n_cells);
+            kl = dbuf<float>(ctx, "cfb_kl", (size_t)S.n_cells);
+            wf = dbuf<float>(ctx, "cfb_wf", (size_t)S.n_cells);
+        }
+        if (P == 0 ? !kap || !w : !kh || !kl || !wf) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (batched CF cells)");
+        launch_cfb_fill_separable(precision, S.n_cells, S.nm, S.nb, (const double*)ctx->arena.find("cfb_tF"),
+                                  (const double*)ctx->arena.find("cfb_tg"), (const double*)ctx->arena.find("cfb_tu"),
+                                  (const double*)ctx->arena.find("cfb_tv"), kap, w, kh, kl, wf, ctx->stream);
+        CKLAUNCH();
+        S.have[P] = true;
+    }
+    return SGL_OK;
+}
+
+void cfb_enqueue(sgl_ctx* ctx, int precision, const CfbRun& R) {
+    CfbState& S = *ctx->cfb;
+    launch_cfb_persistent(precision, R.kt, R.ctas, (const CfbInst*)ctx->arena.find("cfb_inst"), R.items, R.n_items,
+                          R.counter, (const long long*)ctx->arena.find("cfb_pcells"),
                           (const double*)ctx->arena.find("cfb_kap"), (const double*)ctx->arena.find("cfb_w"),
                           (const float*)ctx->arena.find("cfb_kh"), (const float*)ctx->arena.find("cfb_kl"),
                           (const float*)ctx->arena.find("cfb_wf"), (const double*)ctx->arena.find("cfb_vpD"),
                           (const double*)ctx->arena.find("cfb_vpK"), (const double*)ctx->arena.find("cfb_vpw"),
-                          S.nstate, out, ctx->stream);
+                          S.nstate, R.lnphi, ctx->stream, R.parts, S.n_inst,
+                          (const long long*)ctx->arena.find("cfb_koffs"), R.nparts, S.total_k);
+}
+
+sgl_status cfb_launch(sgl_ctx* ctx, int precision, int kt, int cps, const std::vector<int4>* items,
+                      const std::string& tag) {
+    CfbRun R;
+    CKS(cfb_prepare(ctx, precision, kt, cps, items, tag, R));
+    cfb_enqueue(ctx, precision, R);
     CKLAUNCH();
     return SGL_OK;
+}
+
+// The launch shape used when none was tuned: every resident CTA, 64 k-points per item in mixed precision (two warps wait
+// at the barriers of a plane's few cells; 41 gauss and vp instances: step 19.4 ms, 128 wide 19.6; planes at 128 nodes
+// the same within 2%), 128 in FP64.  Timing all shapes on first use, as this did, cost 0.6 s per context.
+void cfb_default_shape(sgl_ctx* ctx, int precision) {
+    CfbState& S = *ctx->cfb;
+    const int P = precision == SGL_FP64 ? 0 : 1;
+    S.kt[P] = P == 1 ? 64 : 128;
+    S.cps[P] = std::max(1, cfb_resident_ctas(precision, S.kt[P]));
+    S.tuned[P] = true;
 }
 
 // The launch shape.  FP64 (the parity path, whose FP64 pipe makes every term slow here) takes a fixed
@@ -106,17 +195,17 @@ sgl_status cfb_tune(sgl_ctx* ctx, int precision) {
     double best = 1e300;
     for (int kt : {64, 128, 256}) {
         const int res = cfb_resident_ctas(precision, kt);
-        std::vector<int2> items = cfb_items(S, kt, sample);
+        std::vector<int4> items = cfb_items(S, kt, sample, {});
         if (istride > 1) {
-            std::vector<int2> sub;
+            std::vector<int4> sub;
             for (size_t q = 0; q < items.size(); q += istride) sub.push_back(items[q]);
             items.swap(sub);
         }
         for (int cps : {1, 2, 4, 8, 16}) {
             if (cps > res) continue;
-            CKS(cfb_launch(ctx, precision, kt, cps, items, "tune"));       // warm
+            CKS(cfb_launch(ctx, precision, kt, cps, &items, "tune"));       // warm
             cudaEventRecord(a, ctx->stream);
-            CKS(cfb_launch(ctx, precision, kt, cps, items, "tune"));
+            CKS(cfb_launch(ctx, precision, kt, cps, &items, "tune"));
             cudaEventRecord(b, ctx->stream);
             CK(cudaEventSynchronize(b));
             float ms = 0.f;
@@ -279,17 +368,15 @@ sgl_status sgl_cfb_set_separable(sgl_ctx* ctx, int nm, int nb, const double* F, 
     DBUF(d_g, double, "cfb_tg", nb);
     DBUF(d_u, double, "cfb_tu", (long long)n_planes * nm);
     DBUF(d_v, double, "cfb_tv", (long long)n_planes * nm);
-    DBUF(d_kap, double, "cfb_kap", nc);
-    DBUF(d_w, double, "cfb_w", nc);
-    DBUF(d_kh, float, "cfb_kh", nc);
-    DBUF(d_kl, float, "cfb_kl", nc);
-    DBUF(d_wf, float, "cfb_wf", nc);
     CKS(upload(ctx, d_F, F, (size_t)per));
     CKS(upload(ctx, d_g, g, (size_t)nb));
     CKS(upload(ctx, d_u, u, (size_t)n_planes * nm));
     CKS(upload(ctx, d_v, v, (size_t)n_planes * nm));
-    launch_cfb_fill_separable(nc, nm, nb, d_F, d_g, d_u, d_v, d_kap, d_w, d_kh, d_kl, d_wf, ctx->stream);
-    CKLAUNCH();
+    // the cells themselves follow in the first solve, in its precision's form
+    CfbState& S = *ctx->cfb;
+    S.nm = nm;
+    S.nb = nb;
+    S.have[0] = S.have[1] = false;
     return sync_stream(ctx);
 }
 
@@ -312,9 +399,8 @@ sgl_status sgl_cfb_lnphi(sgl_ctx* ctx, int precision, double* out) {
     CK(cudaSetDevice(ctx->device));
     CfbState& S = *ctx->cfb;
     const int P = precision == SGL_FP64 ? 0 : 1;
-    if (!S.tuned[P]) CKS(cfb_tune(ctx, precision));
-    const std::vector<int2> items = cfb_items(S, S.kt[P], S.order);
-    CKS(cfb_launch(ctx, precision, S.kt[P], S.cps[P], items, "run"));
+    if (!S.tuned[P]) cfb_default_shape(ctx, precision);
+    CKS(cfb_launch(ctx, precision, S.kt[P], S.cps[P], nullptr, "run"));
     if (out) CK(cudaMemcpyAsync(out, ctx->arena.find("cfb_lnphi"), (size_t)S.total_k * 16, cudaMemcpyDeviceToHost, ctx->stream));
     return sync_stream(ctx);
 }
@@ -331,31 +417,22 @@ sgl_status sgl_cfb_pdf(sgl_ctx* ctx, int precision, const double* lnmu, int n_ln
     for (const CfbInst& I : S.inst)
         if (I.k0 != 0.0 || I.geom) return fail(ctx, SGL_ERR_VALUE, "sgl_cfb_pdf: the inversion needs k grids n dk");
     const int P = precision == SGL_FP64 ? 0 : 1;
-    if (!S.tuned[P]) CKS(cfb_tune(ctx, precision));
+    if (!S.tuned[P]) cfb_default_shape(ctx, precision);
     // every buffer of the step exists before a capture (no allocation inside it)
-    const std::vector<int2> items = cfb_items(S, S.kt[P], S.order);
-    DBUF(d_items, int2, std::string("cfb_items_run") + (P ? "m" : "d"), std::max<size_t>(1, items.size()));
-    DBUF(counter, int, "cfb_counter", 1);
-    DBUF(lnphi, double2, "cfb_lnphi", std::max<long long>(1, S.total_k));
-    void* phi = ctx->arena.get("cfb_phi", (size_t)std::max<long long>(1, S.total_k) * 2 * (P ? 4 : 8));
-    DBUF(d_lnmu, double, "cfb_lnmu", n_lnmu);
-    DBUF(d_P, double, "cfb_P", (long long)S.n_inst * n_lnmu);
+    CfbRun R;
+    CKS(cfb_prepare(ctx, precision, S.kt[P], S.cps[P], nullptr, std::string("run") + (P ? "m" : "d"), R));
+    // (named per precision: a buffer that the other precision's call grows would move under this one's graph)
+    const std::string suffix = P ? "m" : "d";
+    void* phi = ctx->arena.get("cfb_phi_" + suffix, (size_t)std::max<long long>(1, S.total_k) * 2 * (P ? 4 : 8));
+    DBUF(d_lnmu, double, "cfb_lnmu_" + suffix, n_lnmu);
+    DBUF(d_P, double, "cfb_P_" + suffix, (long long)S.n_inst * n_lnmu);
     if (!phi) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (cfb phi)");
-    const int res = cfb_resident_ctas(precision, S.kt[P]);
-    const int ctas = kNumSMs * std::max(1, std::min(S.cps[P], std::max(1, res)));
     const cudaStream_t st = ctx->stream;
     auto enqueue = [&]() {
-        launch_cfb_persistent(precision, S.kt[P], ctas, (const CfbInst*)ctx->arena.find("cfb_inst"), d_items,
-                              (int)items.size(), counter, (const long long*)ctx->arena.find("cfb_pcells"),
-                              (const double*)ctx->arena.find("cfb_kap"), (const double*)ctx->arena.find("cfb_w"),
-                              (const float*)ctx->arena.find("cfb_kh"), (const float*)ctx->arena.find("cfb_kl"),
-                              (const float*)ctx->arena.find("cfb_wf"), (const double*)ctx->arena.find("cfb_vpD"),
-                              (const double*)ctx->arena.find("cfb_vpK"), (const double*)ctx->arena.find("cfb_vpw"),
-                              S.nstate, lnphi, st);
-        launch_cfb_pdf(precision, (const CfbInst*)ctx->arena.find("cfb_inst"), S.n_inst, lnphi, S.total_k,
+        cfb_enqueue(ctx, precision, R);
+        launch_cfb_pdf(precision, (const CfbInst*)ctx->arena.find("cfb_inst"), S.n_inst, R.lnphi, S.total_k,
                        (const long long*)ctx->arena.find("cfb_koffs"), phi, d_lnmu, n_lnmu, d_P, st);
     };
-    CKS(upload(ctx, d_items, items.data(), items.size()));
     CKS(upload(ctx, d_lnmu, lnmu, (size_t)n_lnmu));
     const bool reuse = use_graph && S.graph[P] && S.graph_nm[P] == n_lnmu && S.graph_kt[P] == S.kt[P] &&
                        S.graph_cps[P] == S.cps[P];

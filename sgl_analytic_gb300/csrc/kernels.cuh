@@ -147,15 +147,18 @@ struct CfbInst {                          // one instance of the batch
     int geom;                             // 1: the solve's k points are exp(k0 + n dk) (log-spaced)
     double k0;                            // else k0 + n dk (the inversion assumes k0 = 0)
 };
-void launch_cfb_persistent(int precision, int kt, int ctas, const CfbInst* inst, const int2* items, int n_items,
+// items (instance, k tile, part, parts); parts buffer and nparts per instance only when some instance is split
+void launch_cfb_persistent(int precision, int kt, int ctas, const CfbInst* inst, const int4* items, int n_items,
                            int* counter, const long long* plane_cells, const double* kap, const double* w,
                            const float* kh, const float* kl, const float* wf, const double* vp_D, const double* vp_K,
-                           const double* vp_w, int nstate, double2* out, cudaStream_t st);
+                           const double* vp_w, int nstate, double2* out, cudaStream_t st, double2* parts, int n_inst,
+                           const long long* k_offs, const int* nparts, long long total_k);
 void launch_cfb_pdf(int precision, const CfbInst* inst, int n_inst, const double2* lnphi, long long total,
                     const long long* k_offs, void* phi, const double* lnmu, int nm, double* P, cudaStream_t st);
 int cfb_resident_ctas(int precision, int kt);
-void launch_cfb_fill_separable(long long n_cells, int nm, int nb, const double* F, const double* g, const double* u,
-                               const double* v, double* kap, double* w, float* kh, float* kl, float* wf, cudaStream_t st);
+void launch_cfb_fill_separable(int precision, long long n_cells, int nm, int nb, const double* F, const double* g,
+                               const double* u, const double* v, double* kap, double* w, float* kh, float* kl, float* wf,
+                               cudaStream_t st);
 struct SurPlane {                         // one plane of the surrogate sweep
     double s, dz;                         // lensing efficiency, thickness: the plane adds dz H(s k)
     double lnq0, hq;                      // its surrogate nodes ln q_j = lnq0 + j hq
