@@ -23,7 +23,8 @@
 // over the sorted bounds and each state's z is written once (FP64, [shell][state][point]).
 // Phase 2 (k_vp_chain): one thread per point walks the shells: projection, alpha' = K^T alpha (or the
 // stationary weights at s = 0) times exp(z - max Re z), renormalisation by max |alpha|, log scale;
-// FP64 in both precisions.  Thread-private shared memory, no barriers.
+// FP64, thread-private shared memory, no barriers.  The mixed path's chain (k_vp_chain_ff) is the same recursion in
+// float-float.
 #include "kernels.cuh"
 
 namespace sgl {
@@ -326,6 +327,288 @@ k_vp_chain(VpDevice d, const double2* __restrict__ zp, const double2* __restrict
     out_im[o] = atan2(si, sr);
 }
 
+// The chain of the mixed path in float-float on the FP32 pipe.  In FP64 a (point, shell) step is 4608 FMAs of the
+// transition and 48 exponentials and sincos, some 10^4 operations on a pipe of 2 per clock and SM; here the transition
+// takes 12 packed (re, im) FP32 operations per state pair at 64 lanes per clock, e^z about 200 FP32 operations per state, and
+// FP64 stays where z comes in (projection, maximum, the logarithm of the scale).  The state is renormalised by a power of
+// two, which is exact.  CTA: 32 points; phase A a thread per (point, 8 states): z, e^z into shared memory; phase B a thread
+// per (4 states, 2 points): alpha' = K^T alpha, times e^z.  409 x 109 points, 24 shells: 19.7 -> 3.7 ms; ln R differs from the FP64
+// path by the same 6e-12 (1 + |ln R|) as with the FP64 chain.
+constexpr int kCfPts = 32, kCfThreads = 192;
+
+typedef unsigned long long P2;
+__device__ __forceinline__ P2 p2_mul(P2 a, P2 b) { P2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ P2 p2_add(P2 a, P2 b) { P2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ P2 p2_fma(P2 a, P2 b, P2 c) { P2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ P2 p2_sub(P2 a, P2 b, P2 m1) { return p2_fma(b, m1, a); }
+
+__device__ __forceinline__ ff ff_two_sum(float a, float b) {
+    ff r;
+    r.hi = a + b;
+    const float bb = r.hi - a;
+    r.lo = (a - (r.hi - bb)) + (b - bb);
+    return r;
+}
+__device__ __forceinline__ ff ff_quick(float a, float b) { ff r; r.hi = a + b; r.lo = b - (r.hi - a); return r; }   // |a| >= |b|
+__device__ __forceinline__ ff ffx_add(ff a, ff b) {
+    const ff s = ff_two_sum(a.hi, b.hi);
+    return ff_quick(s.hi, s.lo + (a.lo + b.lo));
+}
+__device__ __forceinline__ ff ffx_mul(ff a, ff b) {
+    const float p = a.hi * b.hi;
+    return ff_quick(p, fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, fmaf(a.hi, b.hi, -p))));
+}
+__device__ __forceinline__ ff ff_neg(ff a) { a.hi = -a.hi; a.lo = -a.lo; return a; }
+
+// x - q C, C = c1 + (c2h + c2l), q an integer: q c1 and x.hi - q c1 are exact (c1 of few bits)
+__device__ __forceinline__ ff ff_reduce(ff x, float q, float c1, float c2h, float c2l) {
+    const float r1 = fmaf(-q, c1, x.hi);
+    const float p = q * c2h, e = fmaf(q, c2h, -p);
+    const ff s = ff_two_sum(r1, -p);
+    return ff_quick(s.hi, s.lo + ((x.lo - e) - q * c2l));
+}
+
+// e^x, x <= 0: x = n ln 2 + r, 1 + r + r^2 / 2 + r^3 / 6 in float-float, the rest (6e-4 of the value) in FP32
+__device__ __forceinline__ ff ff_exp(ff x) {
+    ff z = {0.f, 0.f};
+    if (x.hi < -86.f) return z;
+    const float n = rintf(x.hi * 1.44269504088896341f);
+    const ff r = ff_reduce(x, n, 0.693359375f, -2.12194442e-4f, 1.64659497e-12f);
+    float t = fmaf(r.hi, 1.f / 3628800.f, 1.f / 362880.f);
+    t = fmaf(r.hi, t, 1.f / 40320.f);
+    t = fmaf(r.hi, t, 1.f / 5040.f);
+    t = fmaf(r.hi, t, 1.f / 720.f);
+    t = fmaf(r.hi, t, 1.f / 120.f);
+    t = fmaf(r.hi, t, 1.f / 24.f);
+    const ff r2 = ffx_mul(r, r);
+    const ff sixth = {0.166666672f, -4.96705388e-9f};
+    const ff r3 = ffx_mul(ffx_mul(r2, r), sixth);
+    const ff h = {0.5f * r2.hi, 0.5f * r2.lo}, one = {1.f, 0.f};
+    ff v = ff_quick(r3.hi, fmaf(r2.hi * r2.hi, t, r3.lo));
+    v = ffx_add(h, v);
+    v = ffx_add(r, v);
+    v = ffx_add(one, v);
+    const float sc = __int_as_float(((int)n + 127) << 23);           // n >= -125
+    v.hi *= sc;
+    v.lo *= sc;
+    return v;
+}
+
+// sin x and cos x, |x| <= 2e4: x = q pi/2 + r; r, r^3 / 6 and 1, r^2 / 2, r^4 / 24 in float-float, the rest in FP32
+__device__ __forceinline__ void ff_sincos(ff x, ff& s, ff& c) {
+    const float q = rintf(x.hi * 0.636619772367581343f);
+    const ff r = ff_reduce(x, q, 1.5703125f, 4.83826792e-4f, 2.56334407e-12f);
+    const ff r2 = ffx_mul(r, r), r3 = ffx_mul(r2, r), r4 = ffx_mul(r2, r2);
+    const ff sixth = {0.166666672f, -4.96705388e-9f}, c24 = {0.0416666679f, -1.24176347e-9f}, one = {1.f, 0.f};
+    float t = fmaf(r2.hi, -1.f / 39916800.f, 1.f / 362880.f);
+    t = fmaf(r2.hi, t, -1.f / 5040.f);
+    t = fmaf(r2.hi, t, 1.f / 120.f);
+    const ff a = ff_neg(ffx_mul(r3, sixth));
+    ff sn = ffx_add(r, ff_quick(a.hi, fmaf(r3.hi * r2.hi, t, a.lo)));
+    t = fmaf(r2.hi, -1.f / 3628800.f, 1.f / 40320.f);
+    t = fmaf(r2.hi, t, -1.f / 720.f);
+    const ff b = ffx_mul(r4, c24), h = {-0.5f * r2.hi, -0.5f * r2.lo};
+    ff cs = ffx_add(h, ff_quick(b.hi, fmaf(r4.hi * r2.hi, t, b.lo)));
+    cs = ffx_add(one, cs);
+    const int k = (int)q & 3;
+    s = k & 1 ? cs : sn;
+    c = k & 1 ? sn : cs;
+    if (k & 2) s = ff_neg(s);
+    if ((k + 1) & 2) c = ff_neg(c);
+}
+
+__global__ void k_vp_K_ff(const double* __restrict__ K, long long n, float2* __restrict__ out) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    const ff f = ff_from_double(K[e]);
+    out[e] = make_float2(f.hi, f.lo);
+}
+
+struct ChainShared {
+    float4 alpha[kVpNS][kCfPts];               // (re hi, im hi, re lo, im lo)
+    float4 ez[kVpNS][kCfPts];                  // e^{z - max}
+    float4 K[kVpNS][kVpNS / 2];                // two states: (hi, lo, hi, lo)
+    double red[6][kCfPts][2];
+    double mean[kCfPts][2], mx[kCfPts], scale[kCfPts];
+    unsigned big[kCfPts];
+};
+
+__global__ void __launch_bounds__(kCfThreads, 2)
+k_vp_chain_ff(VpDevice d, const float2* __restrict__ Kff, const double2* __restrict__ zp, const double2* __restrict__ alin,
+              long long NP, int nq, int kb, double* __restrict__ out_re, double* __restrict__ out_im, int npieces) {
+    extern __shared__ __align__(16) unsigned char vsm[];
+    ChainShared& S = *reinterpret_cast<ChainShared*>(vsm);
+    const int t = threadIdx.x, pa = t % kCfPts, ja = t / kCfPts;             // phase A: point, states 8 ja .. 8 ja + 7
+    const int pb = t % 16, jb = 4 * (t / 16);                                // phase B: points pb, pb + 16, states jb .. jb + 3
+    const long long p0 = (long long)blockIdx.x * kCfPts, p = p0 + pa;
+    const bool live = p < NP;
+    if (t < kCfPts) S.scale[t] = 0.0;
+    const P2 m1 = f32x2_pack(-1.f, -1.f);
+    for (int s = 0; s < d.nsh; ++s) {
+        __syncthreads();                       // the previous shell's readers of alpha, K and the reductions are done
+        if (s > 0) {
+            const float4* Ks = reinterpret_cast<const float4*>(Kff + (long long)(s - 1) * kVpNS * kVpNS);
+            for (int e = t; e < kVpNS * kVpNS / 2; e += kCfThreads) (&S.K[0][0])[e] = Ks[e];
+        }
+        // ---- phase A: z with zero stationary mean
+        double zr[8], zi[8];
+        {
+            double2 al = make_double2(0.0, 0.0);
+            if (live)
+                for (int pc = 0; pc < npieces; ++pc) {
+                    const double2 a2 = alin[((long long)pc * d.nsh + s) * NP + p];
+                    al.x += a2.x; al.y += a2.y;
+                }
+            double mr = 0.0, mi = 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int j = 8 * ja + q;
+                double2 zz = make_double2(0.0, 0.0);
+                if (live)
+                    for (int pc = 0; pc < npieces; ++pc) {
+                        const double2 z2 = zp[(((long long)pc * d.nsh + s) * kVpNS + j) * NP + p];
+                        zz.x += z2.x; zz.y += z2.y;
+                    }
+                const double uj = d.u[j], wj = d.w[j];
+                zr[q] = fma(uj, al.x, zz.x);
+                zi[q] = fma(uj, al.y, zz.y);
+                mr = fma(wj, zr[q], mr);
+                mi = fma(wj, zi[q], mi);
+            }
+            S.red[ja][pa][0] = mr;
+            S.red[ja][pa][1] = mi;
+        }
+        __syncthreads();
+        if (t < 2 * kCfPts) {
+            const int pp = t >> 1, c = t & 1;
+            double v = 0.0;
+#pragma unroll
+            for (int g = 0; g < 6; ++g) v += S.red[g][pp][c];
+            S.mean[pp][c] = v;
+        }
+        __syncthreads();
+        {
+            const double mr = S.mean[pa][0], mi = S.mean[pa][1];
+            double mx = -1e300;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                zr[q] -= mr;
+                zi[q] -= mi;
+                mx = fmax(mx, zr[q]);
+            }
+            S.red[ja][pa][0] = mx;
+        }
+        __syncthreads();
+        if (t < kCfPts) {
+            double v = S.red[0][t][0];
+#pragma unroll
+            for (int g = 1; g < 6; ++g) v = fmax(v, S.red[g][t][0]);
+            S.mx[t] = v;
+            S.big[t] = 0u;
+        }
+        __syncthreads();
+        {
+            const double mx = S.mx[pa];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const ff m = ff_exp(ff_from_double(zr[q] - mx));
+                ff sn, cs;
+                if (fabs(zi[q]) <= 2e4) {
+                    ff_sincos(ff_from_double(zi[q]), sn, cs);
+                } else {
+                    double ds, dc;
+                    sincos(zi[q], &ds, &dc);
+                    sn = ff_from_double(ds);
+                    cs = ff_from_double(dc);
+                }
+                const ff er = ffx_mul(m, cs), ei = ffx_mul(m, sn);
+                S.ez[8 * ja + q][pa] = make_float4(er.hi, ei.hi, er.lo, ei.lo);
+            }
+        }
+        // ---- phase B: alpha' = K^T alpha (the stationary weights at the first shell)
+        P2 gh[4][2], gl[4][2];
+        if (s == 0) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const ff w = ff_from_double(d.w[jb + q]);
+#pragma unroll
+                for (int x = 0; x < 2; ++x) { gh[q][x] = f32x2_pack(w.hi, 0.f); gl[q][x] = f32x2_pack(w.lo, 0.f); }
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) { gh[q][x] = 0ull; gl[q][x] = 0ull; }
+#pragma unroll 2
+            for (int i = 0; i < kVpNS; ++i) {
+                const float4 k01 = S.K[i][jb / 2], k23 = S.K[i][jb / 2 + 1];
+                const float4 a0 = S.alpha[i][pb], a1 = S.alpha[i][pb + 16];
+                const P2 ah[2] = {f32x2_pack(a0.x, a0.y), f32x2_pack(a1.x, a1.y)};
+                const P2 al2[2] = {f32x2_pack(a0.z, a0.w), f32x2_pack(a1.z, a1.w)};
+                const float kh[4] = {k01.x, k01.z, k23.x, k23.z}, kl[4] = {k01.y, k01.w, k23.y, k23.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const P2 h = f32x2_pack(kh[q], kh[q]), nh = f32x2_pack(-kh[q], -kh[q]), l = f32x2_pack(kl[q], kl[q]);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        const P2 pr = p2_mul(h, ah[x]), ne = p2_fma(nh, ah[x], pr);     // product, minus its error
+                        const P2 sum = p2_add(gh[q][x], pr), bb = p2_sub(sum, gh[q][x], m1);
+                        const P2 er = p2_add(p2_sub(gh[q][x], p2_sub(sum, bb, m1), m1), p2_sub(pr, bb, m1));
+                        P2 lo = p2_add(gl[q][x], er);
+                        lo = p2_sub(lo, ne, m1);
+                        lo = p2_fma(l, ah[x], lo);
+                        gl[q][x] = p2_fma(h, al2[x], lo);
+                        gh[q][x] = sum;
+                    }
+                }
+            }
+        }
+        __syncthreads();                       // e^z complete; every reader of alpha is done
+        float4 na[4][2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            float big = 0.f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 h = f32x2_unpack(gh[q][x]), l = f32x2_unpack(gl[q][x]);
+                const ff gr = ff_quick(h.x, l.x), gi = ff_quick(h.y, l.y);
+                const float4 e = S.ez[jb + q][pb + 16 * x];
+                const ff er = {e.x, e.z}, ei = {e.y, e.w};
+                const ff nr = ffx_add(ffx_mul(gr, er), ff_neg(ffx_mul(gi, ei)));
+                const ff ni = ffx_add(ffx_mul(gr, ei), ffx_mul(gi, er));
+                na[q][x] = make_float4(nr.hi, ni.hi, nr.lo, ni.lo);
+                big = fmaxf(big, fabsf(nr.hi) + fabsf(ni.hi));
+            }
+            atomicMax(&S.big[pb + 16 * x], __float_as_uint(big));
+        }
+        __syncthreads();
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            // 2^-ex with the largest modulus in [1/2, 2): exact
+            const int ex = (int)(S.big[pb + 16 * x] >> 23) - 126;
+            const float sc = __int_as_float((127 - max(-126, min(126, ex))) << 23);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 v = na[q][x];
+                S.alpha[jb + q][pb + 16 * x] = make_float4(v.x * sc, v.y * sc, v.z * sc, v.w * sc);
+            }
+        }
+        if (t < kCfPts) S.scale[t] += S.mx[t] + max(-126, min(126, (int)(S.big[t] >> 23) - 126)) * 0.6931471805599453;
+    }
+    __syncthreads();
+    if (t < kCfPts && live) {
+        double sr = 0.0, si = 0.0;
+        for (int j = 0; j < kVpNS; ++j) {
+            const float4 v = S.alpha[j][t];
+            sr += (double)v.x + (double)v.z;
+            si += (double)v.y + (double)v.w;
+        }
+        const long long o = (long long)kb * nq + p;
+        out_re[o] = S.scale[t] + 0.5 * log(sr * sr + si * si);
+        out_im[o] = atan2(si, sr);
+    }
+}
+
 // The same chain for few points (the k-reach probe lines): one CTA per point, one thread per state.
 // The per-state work (mat-vec over i in the same order, exp, sincos, normalisation) runs in
 // parallel; the two ordered sums (the projection's weighted mean, the final state sum) stay on
@@ -442,7 +725,7 @@ int vp_pieces(int nsh, int rows, int nq) {
 }
 
 void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, const double* qv, int nq, void* tables,
-                   double2* zbuf, int rows_per_pass, double* out_re, double* out_im, cudaStream_t st, int npieces) {
+                   double2* zbuf, int rows_per_pass, double* out_re, double* out_im, cudaStream_t st, int npieces, float2* Kff) {
     const long long tot = (long long)d.U * (nk + nq);
     const size_t es = precision == SGL_FP64 ? 8 : 4;
     void* e = tables;
@@ -456,6 +739,11 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
     }
     const size_t chain_smem = (4 * (size_t)kVpNS * kChPts + (size_t)kVpNS * kVpNS) * sizeof(double);
     cudaFuncSetAttribute(k_vp_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chain_smem);
+    if (Kff) {
+        const long long nK = (long long)(d.nsh - 1) * kVpNS * kVpNS;
+        if (nK > 0) { k_vp_K_ff<<<ceil_div(nK, 256), 256, 0, st>>>(d.K, nK, Kff); SGL_COUNT(1); }
+        cudaFuncSetAttribute(k_vp_chain_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChainShared));
+    }
     for (int kb = 0; kb < nk; kb += rows_per_pass) {
         const int nkc = nk - kb < rows_per_pass ? nk - kb : rows_per_pass;
         const long long NP = (long long)nkc * nq;
@@ -473,6 +761,10 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
         }
         if (NP <= 4LL * kNumSMs) {
             k_vp_chain_small<<<(unsigned)NP, kChSmallThreads, 0, st>>>(d, zp, al, NP, nq, kb, out_re, out_im, npieces);
+            SGL_COUNT(1);
+        } else if (Kff) {
+            k_vp_chain_ff<<<ceil_div(NP, kCfPts), kCfThreads, sizeof(ChainShared), st>>>(d, Kff, zp, al, NP, nq, kb, out_re,
+                                                                                         out_im, npieces);
             SGL_COUNT(1);
         } else {
             k_vp_chain<<<ceil_div(NP, kChPts), kChPts, chain_smem, st>>>(d, zp, al, NP, nq, kb, out_re, out_im, npieces);
