@@ -23,9 +23,9 @@ void unwrap_line(double* p, int n, long long stride) {
 sgl_status vp_lnR_device(sgl_ctx* ctx, int precision, const double* d_kv, int nk, const double* d_qv, int nq,
                          double* d_re, double* d_im) {
     const VpDevice& D = ctx->vpd;
-    void* tables = ctx->arena.get("vp_tables", vp_table_bytes(precision, D.U, nk, nq));
+    void* tables = ctx->arena.get("vp_tables", vp_table_bytes(precision, D.U, nk, nq, D.nruns));
     const int rows = vp_rows_per_pass(D.nsh, nk, nq, (size_t)8 << 30);
-    const int pieces = rows == nk ? vp_pieces(D.nsh, rows, nq) : 1;     // split runs only in a single pass
+    const int pieces = rows == nk ? vp_pieces(precision, D.nsh, rows, nq) : 1;     // split runs only in a single pass
     void* zb = ctx->arena.get("vp_z", (size_t)D.nsh * 49 * 16 * (size_t)rows * nq * pieces);
     if (!tables || !zb) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (vp)");
     const double pts = (double)nk * nq;

@@ -16,7 +16,7 @@
 // z_s = z_partial - E_w[z_partial] exactly, and that projection also removes the common-mode part
 // of the rounding error (what keeps the mixed path within 1e-8 of FP64).
 //
-// Phase 1 (k_vp_z): one CTA per (shell, 16 k x 32 q tile); each thread owns 2 x 2 points.  Cells of
+// Phase 1 (k_vp_z; on a grid of points in mixed precision k_vp_z_mixed, below): one CTA per (shell, 16 k x 32 q tile); each thread owns 2 x 2 points.  Cells of
 // a run stream through shared memory in chunks of 32 (table rows e[u][k], (J, J - 1)[u][q] gathered
 // by cell index, coalesced along k / q); per point 4 FMAs + 2 for F.  Mixed: FP32 chunk sums folded
 // into float-float run totals (TwoSum); FP64: FP64 throughout.  Run totals go to FP64 running sums
@@ -60,6 +60,17 @@ __global__ void k_vp_tables(const double* __restrict__ ku, const double* __restr
         Jt[r].x = (TT)(1.0 + jm);
         Jt[r].y = (TT)jm;
     }
+}
+
+__device__ __forceinline__ unsigned long long vz_add(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long vz_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
 // hi + lo += p  (Knuth TwoSum; no FMA contraction applies to additions)
@@ -238,6 +249,276 @@ k_vp_z(VpDevice d, const typename V2<TT>::T* __restrict__ e, const typename V2<T
         if (live[P]) alin[(long long)s * NP + pidx[P]] = make_double2(ALr[P], ALi[P]);
 }
 
+// ---- phase 1 of the mixed path on a grid of points
+// F splits into e_c(k) J_c(q), of both axes, and J_c(q) - 1, of k_gamma alone: the second part of every run is summed
+// once per q (k_vp_jm), and per (cell, point) only two packed FMAs remain, J times (w a e_re, w a e_im) and
+// (w b e_re, w b e_im), the four products formed once per (cell, k) while staging (k_vp_z forms F and needs six scalar
+// ones).  CTA: 16 k x 112 q of one shell (or a piece of its runs), 2 k x 7 q per thread, so that a cell costs a warp five
+// shared-memory reads to 28 FMAs; FP32 sums over 32 cells, compensated (Kahan) over the run; the sums over the sorted
+// bounds live in local memory, touched once per run.  Bound by the FP32 pipe; 409 x 109 points, 0.77 M cells:
+// 21.9 -> 9.1 ms (issue 50% active, two warps per scheduler: the 56 pairs of compensated sums take 112 registers).
+constexpr int kMzK = 16, kMzQ = 112, kMzThreads = 128, kMzCh = 32;
+
+// J0 and J0 - 1 per unique cell with rows padded to whole q tiles (zeros), e as in k_vp_tables
+__global__ void k_vp_tables_mixed(const double* __restrict__ ku, const double* __restrict__ gu, int U,
+                                  const double* __restrict__ kv, int nk, const double* __restrict__ qv, int nq, int nqp,
+                                  float2* __restrict__ e, float* __restrict__ J, float* __restrict__ Jm) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long ne = (long long)U * nk;
+    if (t < ne) {
+        const int u = (int)(t / nk), i = (int)(t % nk);
+        const double ph = kv[i] * ku[u];
+        double s, c;
+        sincos(0.5 * ph, &s, &c);
+        e[t] = make_float2((float)(-2.0 * s * s), (float)(2.0 * s * c));
+    } else if (t < ne + (long long)U * nqp) {
+        const long long r = t - ne;
+        const int u = (int)(r / nqp), j = (int)(r % nqp);
+        const double jm = j < nq ? j0m1_d(qv[j] * gu[u]) : -1.0;
+        J[r] = (float)(1.0 + jm);
+        Jm[r] = j < nq ? (float)jm : 0.f;
+    }
+}
+
+// per run, part of its cells and q: sum_c (w a, w b)_c (J_c(q) - 1), FP32 over 32 cells, FP64 over the part; then the
+// parts in order
+constexpr int kJmParts = 16;
+__global__ void __launch_bounds__(128) k_vp_jm(VpDevice d, const float* __restrict__ Jm, int nqp, double2* __restrict__ part) {
+    const int r = blockIdx.x, q = blockIdx.z * 128 + threadIdx.x;
+    if (q >= nqp) return;
+    const long long n0 = d.run_cell[r], n1 = d.run_cell[r + 1];
+    const long long per = ((n1 - n0 + kJmParts - 1) / kJmParts + 31) / 32 * 32;
+    const long long c0 = min(n1, n0 + blockIdx.y * per), c1 = min(n1, c0 + per);
+    double a = 0.0, b = 0.0;
+    for (long long base = c0; base < c1; base += 32) {
+        const int cnt = (int)min(32LL, c1 - base);
+        float pa = 0.f, pb = 0.f;
+#pragma unroll 8
+        for (int c = 0; c < cnt; ++c) {
+            const float2 w = d.wabf[base + c];
+            const float j = Jm[(long long)d.cu[base + c] * nqp + q];
+            pa = fmaf(w.x, j, pa);
+            pb = fmaf(w.y, j, pb);
+        }
+        a += (double)pa;
+        b += (double)pb;
+    }
+    part[((long long)blockIdx.y * d.nruns + r) * nqp + q] = make_double2(a, b);
+}
+
+__global__ void k_vp_jm_sum(const double2* __restrict__ part, long long n, double2* __restrict__ out) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    double a = 0.0, b = 0.0;
+    for (int p = 0; p < kJmParts; ++p) { const double2 v = part[p * n + e]; a += v.x; b += v.y; }
+    out[e] = make_double2(a, b);
+}
+
+__global__ void __launch_bounds__(kMzThreads, 2)
+k_vp_z_mixed(VpDevice d, const float2* __restrict__ e, const float* __restrict__ J, const double2* __restrict__ jm, int nk,
+             int nq, int nqp, int kb, int nkc, double2* __restrict__ zp, double2* __restrict__ alin, long long NP, int npieces) {
+    __shared__ __align__(16) float s_J[2][kMzCh][kMzQ];
+    __shared__ __align__(16) float4 s_we[2][kMzCh][kMzK];
+    __shared__ int s_cu[4][kMzCh];             // unique-cell indices, two chunks ahead of the sums
+    const int s = blockIdx.z / npieces, piece = blockIdx.z % npieces;
+    zp += (long long)piece * d.nsh * kVpNS * NP;
+    alin += (long long)piece * d.nsh * NP;
+    const int q0 = blockIdx.x * kMzQ, k0 = kb + blockIdx.y * kMzK, kend = kb + nkc;
+    const int t = threadIdx.x, lane = t & 31, tq = lane & 15;
+    const int kl = (t >> 5) * 4 + (lane >> 4) * 2;                        // the thread's k: k0 + kl, + 1
+    // its q: q0 + 4 tq + 0..3, 64 + 2 tq + 0..1, 96 + tq
+    auto q_of = [&](int i) { return q0 + (i < 4 ? 4 * tq + i : (i < 6 ? 64 + 2 * tq + (i - 4) : 96 + tq)); };
+    // sums over the bounds (A, B anchored at 0, linear A; re, im) in local memory: the opaque offset keeps them there
+    double st[14][6];
+    int z;
+    asm volatile("mov.u32 %0, 0;" : "=r"(z));
+#pragma unroll 1
+    for (int P = 0; P < 14; ++P)
+#pragma unroll 1
+        for (int v = 0; v < 6; ++v) st[P + z][v + z] = 0.0;
+    int jcur = 0;
+    auto emit_to = [&](int jend) {
+        for (; jcur < jend; ++jcur) {
+            const double uj = d.u[jcur];
+            double2* row = zp + ((long long)s * kVpNS + jcur) * NP;
+#pragma unroll 1
+            for (int P = 0; P < 14; ++P) {
+                const int k = k0 + kl + P / 7, q = q_of(P % 7);
+                const double* a = st[P + z];
+                if (k < kend && q < nq)
+                    row[(long long)(k - kb) * nq + q] = make_double2(fma(uj, a[0], a[2]), fma(uj, a[1], a[3]));
+            }
+        }
+    };
+    // the piece's cells: an equal part of the shell's (a run may span pieces: its contribution is additive), and the runs
+    // that hold them
+    const int rs0 = d.sh_run[s], rs1 = d.sh_run[s + 1];
+    const long long sc0 = d.run_cell[rs0], sn = d.run_cell[rs1] - sc0;
+    const long long cb = sc0 + sn * piece / npieces, ce = sc0 + sn * (piece + 1) / npieces;
+    int r0 = rs0, r1 = rs1;
+    while (r0 < r1 && d.run_cell[r0 + 1] <= cb) ++r0;
+    while (r1 > r0 && d.run_cell[r1 - 1] >= ce) --r1;
+    auto first = [&](int r) { return max(cb, d.run_cell[r]); };
+    auto end = [&](int r) { return min(ce, d.run_cell[r + 1]); };
+    // chunks of at most 32 cells that never straddle a run; (r, base) of the chunk after a given one
+    auto next = [&](int& r, long long& base) {
+        base += kMzCh;
+        if (base >= end(r) && ++r < r1) base = first(r);
+    };
+    // staging: the indices of a chunk's cells (slot), then, one chunk later, its J by asynchronous 16-byte copies and its
+    // e and weights into registers, whose products `place` writes
+    auto fetch_cu = [&](int slot, int r, long long base) {
+        if (r < r1 && t < kMzCh) {
+            const bool ok = base + t < end(r);
+            const uint32_t sa = (uint32_t)__cvta_generic_to_shared(&s_cu[slot][t]);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"(sa), "l"(ok ? d.cu + base + t : d.cu), "r"(ok ? 4 : 0) : "memory");
+        }
+    };
+    float2 pe[4], pw[4];
+    auto fetch = [&](int buf, int slot, int r, long long base) {
+        const int cnt = (int)min((long long)kMzCh, end(r) - base);
+#pragma unroll
+        for (int x = 0; x < kMzCh * kMzQ / 4 / kMzThreads; ++x) {
+            const int idx = t + x * kMzThreads, c = idx / (kMzQ / 4), o = (idx % (kMzQ / 4)) * 4;
+            const bool ok = c < cnt;
+            cp_async<16>(&s_J[buf][c][o], ok ? (const void*)(J + (long long)s_cu[slot][c] * nqp + q0 + o) : (const void*)J, ok);
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int idx = t + x * kMzThreads, c = idx / kMzK, k = k0 + idx % kMzK;
+            const bool ok = c < cnt && k < kend;
+            pe[x] = ok ? e[(long long)s_cu[slot][c] * nk + k] : make_float2(0.f, 0.f);
+            pw[x] = ok ? d.wabf[base + c] : make_float2(0.f, 0.f);
+        }
+    };
+    auto place = [&](int buf) {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int idx = t + x * kMzThreads;
+            s_we[buf][idx / kMzK][idx % kMzK] =
+                make_float4(pw[x].x * pe[x].x, pw[x].x * pe[x].y, pw[x].y * pe[x].x, pw[x].y * pe[x].y);
+        }
+    };
+    const unsigned long long m1 = f32x2_pack(-1.f, -1.f);
+    int buf = 0, slot = 0;                     // the chunk being summed: its buffers, its slot of s_cu
+    int rn = r0, r2 = r0;                      // the next chunk, and the one after it
+    long long bn = 0, b2 = 0;
+    if (r0 < r1) {
+        bn = b2 = first(r0);
+        fetch_cu(0, r0, bn);
+        next(r2, b2);
+        fetch_cu(1, r2, b2);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+        fetch(0, 0, r0, bn);
+        cp_async_commit();
+        place(0);
+        cp_async_wait<0>();
+        __syncthreads();
+        rn = r2; bn = b2;
+    }
+    for (int r = r0; r < r1; ++r) {
+        const long long c0 = first(r), c1 = end(r);
+        unsigned long long hi[2][7][2], lo[2][7][2];                       // (k, q, a or b): (re, im), value hi - lo
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int i = 0; i < 7; ++i)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) { hi[x][i][v] = 0ull; lo[x][i][v] = 0ull; }
+        for (long long base = c0; base < c1; base += kMzCh) {
+            const int cnt = (int)min((long long)kMzCh, c1 - base);
+            const bool more = rn < r1;
+            if (more) {
+                fetch(buf ^ 1, (slot + 1) & 3, rn, bn);
+                r2 = rn; b2 = bn;
+                next(r2, b2);
+                fetch_cu((slot + 2) & 3, r2, b2);
+                cp_async_commit();
+            }
+            unsigned long long p[2][7][2];
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int i = 0; i < 7; ++i)
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) p[x][i][v] = 0ull;
+#pragma unroll 2
+            for (int c = 0; c < cnt; ++c) {
+                const float4 j4 = *reinterpret_cast<const float4*>(&s_J[buf][c][4 * tq]);
+                const float2 j2 = *reinterpret_cast<const float2*>(&s_J[buf][c][64 + 2 * tq]);
+                const float jv[7] = {j4.x, j4.y, j4.z, j4.w, j2.x, j2.y, s_J[buf][c][96 + tq]};
+                const float4 w0 = s_we[buf][c][kl], w1 = s_we[buf][c][kl + 1];
+                const unsigned long long wv[2][2] = {{f32x2_pack(w0.x, w0.y), f32x2_pack(w0.z, w0.w)},
+                                                     {f32x2_pack(w1.x, w1.y), f32x2_pack(w1.z, w1.w)}};
+#pragma unroll
+                for (int i = 0; i < 7; ++i) {
+                    const unsigned long long j = f32x2_pack(jv[i], jv[i]);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        f32x2_fma(p[x][i][0], j, wv[x][0]);
+                        f32x2_fma(p[x][i][1], j, wv[x][1]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int i = 0; i < 7; ++i)
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        // Kahan: y = p - lo, sum = hi + y, lo = (sum - hi) - y
+                        const unsigned long long y = vz_fma(lo[x][i][v], m1, p[x][i][v]);
+                        const unsigned long long sum = vz_add(hi[x][i][v], y);
+                        lo[x][i][v] = vz_fma(y, m1, vz_fma(hi[x][i][v], m1, sum));
+                        hi[x][i][v] = sum;
+                    }
+            if (more) {
+                place(buf ^ 1);
+                cp_async_wait<0>();
+            }
+            __syncthreads();
+            buf ^= 1;
+            slot = (slot + 1) & 3;
+            rn = r2; bn = b2;
+        }
+        const int kind = d.run_kind[r], bound = d.run_bound[r];
+        const double ub = d.u[bound];
+        const bool whole = c0 == d.run_cell[r];            // the piece with the run's first cell adds its J - 1 sums
+        if (kind == 1) emit_to(bound);                     // left: states >= lo, anchored at u_lo
+        else if (kind == 2) emit_to(bound + 1);            // right: as in k_vp_z
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int i = 0; i < 7; ++i) {
+                double* a = st[x * 7 + i + z];
+                const float2 ha = f32x2_unpack(hi[x][i][0]), la = f32x2_unpack(lo[x][i][0]);
+                const float2 hb = f32x2_unpack(hi[x][i][1]), lb = f32x2_unpack(lo[x][i][1]);
+                const double2 jq = whole ? jm[(long long)r * nqp + q_of(i)] : make_double2(0.0, 0.0);
+                const double Ar = ((double)ha.x - (double)la.x) + jq.x, Ai = (double)ha.y - (double)la.y;
+                const double Br = ((double)hb.x - (double)lb.x) + jq.y, Bi = (double)hb.y - (double)lb.y;
+                if (kind == 0) {                           // linear: u_j A (intercept dropped)
+                    a[4] += Ar; a[5] += Ai;
+                } else if (kind == 1) {
+                    a[0] += Ar; a[1] += Ai;
+                    a[2] += fma(-ub, Ar, Br); a[3] += fma(-ub, Ai, Bi);
+                } else {
+                    a[4] += Ar; a[5] += Ai;
+                    a[0] -= Ar; a[1] -= Ai;
+                    a[2] += fma(ub, Ar, -Br); a[3] += fma(ub, Ai, -Bi);
+                }
+            }
+    }
+    emit_to(kVpNS);
+#pragma unroll 1
+    for (int P = 0; P < 14; ++P) {
+        const int k = k0 + kl + P / 7, q = q_of(P % 7);
+        if (k < kend && q < nq)
+            alin[(long long)s * NP + (long long)(k - kb) * nq + q] = make_double2(st[P + z][4], st[P + z][5]);
+    }
+}
+
 __global__ void __launch_bounds__(kChPts)
 k_vp_chain(VpDevice d, const double2* __restrict__ zp, const double2* __restrict__ alin, long long NP, int nq, int kb,
            double* __restrict__ out_re, double* __restrict__ out_im, int npieces) {
@@ -338,8 +619,8 @@ constexpr int kCfPts = 32, kCfThreads = 192;
 
 typedef unsigned long long P2;
 __device__ __forceinline__ P2 p2_mul(P2 a, P2 b) { P2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ P2 p2_add(P2 a, P2 b) { P2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ P2 p2_fma(P2 a, P2 b, P2 c) { P2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ P2 p2_add(P2 a, P2 b) { return vz_add(a, b); }
+__device__ __forceinline__ P2 p2_fma(P2 a, P2 b, P2 c) { return vz_fma(a, b, c); }
 __device__ __forceinline__ P2 p2_sub(P2 a, P2 b, P2 m1) { return p2_fma(b, m1, a); }
 
 __device__ __forceinline__ ff ff_two_sum(float a, float b) {
@@ -704,8 +985,15 @@ k_vp_chain_small(VpDevice d, const double2* __restrict__ zp, const double2* __re
     }
 }
 
-size_t vp_table_bytes(int precision, int U, int nk, int nq) {
+// the mixed path's grid kernel pays from a few tiles of points on; the k-reach probe lines keep k_vp_z
+bool vp_mixed_grid(int precision, int nk, int nq) { return precision != SGL_FP64 && nk >= 8 && nq >= 32; }
+static int vp_nqp(int nq) { return ceil_div(nq, kMzQ) * kMzQ; }
+
+size_t vp_table_bytes(int precision, int U, int nk, int nq, int nruns) {
     const size_t es = precision == SGL_FP64 ? 8 : 4;
+    if (vp_mixed_grid(precision, nk, nq))
+        return 8 * (size_t)U * nk + 8 * (size_t)U * vp_nqp(nq) +
+               16 * (size_t)std::max(1, nruns) * vp_nqp(nq) * (kJmParts + 1) + 1024;
     return 2 * es * ((size_t)U * nk + (size_t)U * nq) + 256;
 }
 
@@ -718,7 +1006,12 @@ int vp_rows_per_pass(int nsh, int nk, int nq, size_t z_cap_bytes) {
     return (int)((nk + passes - 1) / passes);
 }
 
-int vp_pieces(int nsh, int rows, int nq) {
+int vp_pieces(int precision, int nsh, int rows, int nq) {
+    if (vp_mixed_grid(precision, rows, nq)) {
+        // two CTAs per SM: at least four waves, so that the last one costs at most a fifth
+        const long long base = (long long)(vp_nqp(nq) / kMzQ) * ceil_div(rows, kMzK) * nsh;
+        return (int)std::max(1LL, std::min(8LL, (4LL * 2 * kNumSMs + base - 1) / base));
+    }
     const long long base = (long long)ceil_div(nq, kZQ) * ceil_div(rows, kZK) * nsh;
     const long long want = 8LL * kNumSMs;                   // CTAs of 128 threads
     return (int)std::max(1LL, std::min(32LL, (want + base - 1) / base));
@@ -730,7 +1023,23 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
     const size_t es = precision == SGL_FP64 ? 8 : 4;
     void* e = tables;
     void* Jt = (char*)tables + 2 * es * (size_t)d.U * nk;
-    if (precision == SGL_FP64) {
+    // mixed grid: e (float2), then the run sums of J - 1 (double2), J and J - 1 with padded rows
+    const bool grid = vp_mixed_grid(precision, nk, nq);
+    const int nqp = vp_nqp(nq);
+    double2* jm = (double2*)(((uintptr_t)tables + 8 * (size_t)d.U * nk + 255) & ~(uintptr_t)255);
+    double2* jm_part = jm + (size_t)std::max(1, d.nruns) * nqp;
+    float* J = (float*)(jm_part + (size_t)std::max(1, d.nruns) * nqp * kJmParts);
+    float* Jm = J + (size_t)d.U * nqp;
+    if (grid) {
+        k_vp_tables_mixed<<<ceil_div((long long)d.U * (nk + nqp), 256), 256, 0, st>>>(d.ku, d.gu, d.U, kv, nk, qv, nq, nqp,
+                                                                                      (float2*)e, J, Jm);
+        SGL_COUNT(1);
+        if (d.nruns > 0) {
+            k_vp_jm<<<dim3(d.nruns, kJmParts, ceil_div(nqp, 128)), 128, 0, st>>>(d, Jm, nqp, jm_part);
+            k_vp_jm_sum<<<ceil_div((long long)d.nruns * nqp, 256), 256, 0, st>>>(jm_part, (long long)d.nruns * nqp, jm);
+            SGL_COUNT(2);
+        }
+    } else if (precision == SGL_FP64) {
         k_vp_tables<double><<<ceil_div(tot, 256), 256, 0, st>>>(d.ku, d.gu, d.U, kv, nk, qv, nq, (double2*)e, (double2*)Jt);
         SGL_COUNT(1);
     } else {
@@ -753,6 +1062,10 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
         if (precision == SGL_FP64) {
             k_vp_z<double><<<g1, kZThreads, 0, st>>>(d, (const double2*)e, (const double2*)Jt, nk, nq, kb, nkc, zp, al, NP,
                                                      npieces);
+            SGL_COUNT(1);
+        } else if (grid) {
+            k_vp_z_mixed<<<dim3(nqp / kMzQ, ceil_div(nkc, kMzK), d.nsh * npieces), kMzThreads, 0, st>>>(
+                d, (const float2*)e, J, jm, nk, nq, nqp, kb, nkc, zp, al, NP, npieces);
             SGL_COUNT(1);
         } else {
             k_vp_z<float><<<g1, kZThreads, 0, st>>>(d, (const float2*)e, (const float2*)Jt, nk, nq, kb, nkc, zp, al, NP,
