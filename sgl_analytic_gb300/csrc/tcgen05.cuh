@@ -109,6 +109,7 @@ __device__ __forceinline__ bool mbar_wait_sleep(uint32_t mbar, uint32_t parity) 
 }
 
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity) {
+    if (mbar_try(mbar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try(mbar, parity))
         if (clock64() - t0 > kTcWaitCycles) return false;
