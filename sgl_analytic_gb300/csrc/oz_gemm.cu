@@ -16,9 +16,9 @@
 //
 // Why: the FP64 pipe does 2 FMA per clock and SM (0.95 TFLOP/s in this engine's SIMT GEMM); 28 digit products of BF16
 // are 28 / 4096 of a clock per FP64 FMA.  Bound by the MMAs' operand reads from L2: a 128 x 64 tile moves 84 KB per
-// 32 k, 900 tensor clocks per 16.  Measured (FP64 SIMT before -> with slicing): sep1 3366 x 580 x 6384 25.2 -> 1.10 ms,
-// Hankel 3366 x 796 x 2687 11.0 -> 0.64, kappa 2400 x 798 x 3366 13.8 -> 0.63, sep2 3366 x 2687 x 446 6.8 -> 0.56, the xi
-// groups (67 GFLOP, K about 300) 70.4 -> 6.5; rms error on such data 6e-17 .. 5e-16 against 6e-16 .. 3e-15.
+// 32 k, 900 tensor clocks per 16.  Measured (FP64 SIMT before -> with slicing): sep1 3366 x 580 x 6384 25.2 -> 1.01 ms,
+// Hankel 3366 x 796 x 2687 11.0 -> 0.53, kappa 2400 x 798 x 3366 13.8 -> 0.57, sep2 3366 x 2687 x 446 6.8 -> 0.40, the xi
+// groups (67 GFLOP, K about 300) 70.4 -> 5.0 (6.5 with row-wise scattered stores and FP64 conversions in the epilogue); rms error on such data 6e-17 .. 5e-16 against 6e-16 .. 3e-15.
 //
 // Layout: operands packed by k_oz_pack as [k block of 32][digit][row][64 B] in the canonical K-major core-matrix
 // layout (as tc_gemm.cu), so that one bulk copy moves a tile's digit.  One CTA per 128 x 64 tile: the seven
@@ -42,7 +42,7 @@ constexpr int kOzStageBytes = kOzS * (kOzABytes + kOzBBytes);               // 8
 constexpr int kOzBarOff = kOzStages * kOzStageBytes;
 constexpr int kOzNBar = 2 * kOzStages + 3;                                  // full, empty, acc full, acc empty, done
 constexpr int kOzSmem = kOzBarOff + 8 * kOzNBar + 32;
-constexpr int kOzScaleRows = 256, kOzScaleK = 128;
+constexpr int kOzScaleRows = 256, kOzScaleK = 64;
 
 namespace {
 
@@ -84,13 +84,16 @@ __global__ void __launch_bounds__(256) k_oz_scale(const OzPackDesc* __restrict__
         const int r = r0 + threadIdx.x;
         if (r >= d.R) return;
         int e = 0;
+#pragma unroll 16
         for (int k = k0; k < k1; ++k)
             e = max(e, exponent(d.X[(long long)r * d.x_rs + (long long)k * d.x_cs], s_shift[k - k0]));
         if (e > 0) atomicMax(scale + d.scale_off + r, e);
     } else {                                                  // rows contiguous along k: a warp per row
         const int lane = threadIdx.x & 31;
+#pragma unroll 4
         for (int r = r0 + (threadIdx.x >> 5); r < min(d.R, r0 + kOzScaleRows); r += 8) {
             int e = 0;
+#pragma unroll 4
             for (int k = k0 + lane; k < k1; k += 32) e = max(e, exponent(d.X[(long long)r * d.x_rs + k], s_shift[k - k0]));
             e = __reduce_max_sync(0xffffffffu, e);
             if (lane == 0 && e > 0) atomicMax(scale + d.scale_off + r, e);
@@ -140,6 +143,36 @@ __global__ void __launch_bounds__(256) k_oz_pack(const OzPackDesc* __restrict__ 
         *reinterpret_cast<uint4*>(out + (long long)s * d.Rpad * 64) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
 }
 
+// hi 2^24 + lo as a double, rounded to nearest even, times 2^(e - 2106): 2^48 of the digits' weights and 2^(e - 1077) of
+// the two operands' integers, e their largest biased exponents.  On the integer pipe (an FP64 instruction, 64-bit
+// conversions included, holds a scheduler for 64 cycles, also where its result is not selected) and without a branch, so
+// that several outputs' chains interleave.  In the rare range outside the normal numbers: the unscaled value, *odd.
+__device__ __forceinline__ double oz_value(long long hi, long long lo, int e, bool* odd) {
+    // magnitude H 2^24 + L, L < 2^24
+    hi += lo >> 24;
+    const bool neg = hi < 0;
+    unsigned int L = (unsigned int)lo & 0xffffffu;
+    unsigned long long H = (unsigned long long)(neg ? ~hi : hi);
+    H += neg && L == 0 ? 1 : 0;
+    L = neg ? (0x1000000u - L) & 0xffffffu : L;
+    const bool low = H == 0;
+    H = low ? L : H;
+    L = low ? 0u : L;
+    const int top = low ? 63 : 87, lz = min(__clzll(H), 63);          // top: exponent of H's bit 63
+    const unsigned long long l40 = (unsigned long long)L << 40;
+    const unsigned long long x = (H << lz) | ((l40 >> 1) >> (63 - lz));
+    const unsigned int rest = (unsigned int)(x & 0x3ff) | (unsigned int)((l40 << lz) != 0);
+    unsigned long long m = x >> 11;                                   // 53 bits
+    m += ((unsigned int)x >> 10) & ((rest != 0 ? 1u : 0u) | (unsigned int)m) & 1u;
+    const int E = top - lz + 1023;                                    // biased exponent before the scale
+    int s = e - 2106;
+    const bool normal = E + s > 0 && E + s < 0x7fe;
+    *odd = !normal && H != 0;
+    s = normal ? s : 0;
+    const long long v = (((long long)(E + s - 1) << 52) + (long long)m) | (neg ? (long long)(1ULL << 63) : 0);
+    return __longlong_as_double(H == 0 ? 0 : v);
+}
+
 __global__ void __launch_bounds__(kOzThreads, 1)
 k_oz_gemm(const OzGemmDesc* __restrict__ descs, int nprob, const unsigned char* __restrict__ packed,
           const int* __restrict__ scale, int* __restrict__ err) {
@@ -154,7 +187,11 @@ k_oz_gemm(const OzGemmDesc* __restrict__ descs, int nprob, const unsigned char* 
     volatile int* s_used = (volatile int*)(tsm + kOzBarOff + 8 * kOzNBar + 12);      // k blocks the MMAs took
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = blockIdx.x;
-    const OzGemmDesc d = descs[find_desc(descs, nprob, tile, [](const OzGemmDesc& x) { return (long long)x.tile_begin; })];
+    // the last problem that begins at or before the tile: counted by all threads, one round trip to memory
+    int before = 0;
+    for (int p0 = 0; p0 < nprob; p0 += kOzThreads)
+        before += __syncthreads_count(p0 + tid < nprob && descs[p0 + tid].tile_begin <= tile);
+    const OzGemmDesc d = descs[before - 1];
     const int local = tile - d.tile_begin;
     const int i0 = (local / d.tiles_n) * kOzBM, j0 = (local % d.tiles_n) * kOzBN;
     const int nkb = (d.K + kOzKB - 1) / kOzKB;
@@ -237,6 +274,7 @@ k_oz_gemm(const OzGemmDesc* __restrict__ descs, int nprob, const unsigned char* 
     } else {
         // hi = sum_d<4 D_d 256^(3 - d), lo = sum_d>=4 D_d 256^(6 - d): 64-bit integers per output
         constexpr int kCols = kOzBN / 2;
+        static_assert(kCols == 32, "a lane per column of a warp's outputs");
         long long hi[kCols], lo[kCols];
 #pragma unroll
         for (int c = 0; c < kCols; ++c) { hi[c] = 0; lo[c] = 0; }
@@ -264,29 +302,44 @@ k_oz_gemm(const OzGemmDesc* __restrict__ descs, int nprob, const unsigned char* 
             if (lane == 0) mbar_arrive(acce);
         }
         if (!ok) *s_fail = 1;
-        const int gi = i0 + (warp & 3) * 32 + lane, jb = j0 + (warp >> 2) * kCols;
-        if (ok && gi < d.M) {
-            const int ea = scale[d.sa_off + gi];
-            const bool scaled = d.alpha != 1.0;
-            double* C = d.C + (long long)gi * d.ldc;
+        // through shared memory (the stages are free: every product has been taken), each warp its own 32 rows, so that
+        // C is written, and read for beta, along its rows
+        if (ok) {
+            const int r0 = i0 + (warp & 3) * 32, j = j0 + (warp >> 2) * kCols + lane;
+            double* s_out = (double*)tsm + warp * 32 * (kCols + 1);
+            const int ea = r0 + lane < d.M ? scale[d.sa_off + r0 + lane] : 0;
+            const int ebs = j < d.N ? scale[d.sb_off + j] : 0;
+            uint32_t odd = 0;                                        // outputs left unscaled, a bit per column
 #pragma unroll
             for (int c = 0; c < kCols; ++c) {
-                const int gj = jb + c;
-                if (gj < d.N) {
-                    const int eb = scale[d.sb_off + gj];
-                    // 2^48 of the weights, 2^(e - 1077) of each operand's integers
-                    // (FP64 instructions count here: 8192 outputs at 2 per clock; the scaling is an integer addition)
-                    double v = fma((double)hi[c], 16777216.0, (double)lo[c]);
-                    const int sh = ea + eb - 2 * kOzBias - 2106;
-                    const int ex = (__double2hiint(v) >> 20) & 0x7ff;
-                    if (ex != 0) {
-                        if (ex + sh > 0 && ex + sh < 0x7ff) v = __hiloint2double(__double2hiint(v) + (sh << 20), __double2loint(v));
-                        else v = scalbn(v, sh);
+                bool o;
+                s_out[lane * (kCols + 1) + c] = oz_value(hi[c], lo[c], ea + __shfl_sync(0xffffffffu, ebs, c) - 2 * kOzBias, &o);
+                odd |= (uint32_t)o << c;
+            }
+            if (__any_sync(0xffffffffu, odd != 0 || ea >= kOzNan || ebs >= kOzNan))
+                for (int c = 0; c < kCols; ++c) {
+                    const int eb = __shfl_sync(0xffffffffu, ebs, c);
+                    double* o = s_out + lane * (kCols + 1) + c;
+                    if (odd >> c & 1) *o = scalbn(*o, ea + eb - 2 * kOzBias - 2106);
+                    if (ea >= kOzNan || eb >= kOzNan) *o = __longlong_as_double(0x7ff8000000000000LL);
+                }
+            __syncwarp();
+            const int nr = j < d.N ? min(32, d.M - r0) : 0;
+            double* C = d.C + (long long)r0 * d.ldc + j;
+            if (d.alpha == 1.0 && d.beta == 0.0) {
+                // a loop of its own: FP64 instructions whose results are not selected take their 64 cycles all the same
+#pragma unroll 8
+                for (int r = 0; r < nr; ++r) C[r * d.ldc] = s_out[r * (kCols + 1) + lane];
+            } else {
+                for (int rb = 0; rb < nr; rb += 8) {                 // eight rows' loads in flight
+                    double c[8];
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) c[r] = d.beta != 0.0 && rb + r < nr ? C[(rb + r) * d.ldc] : 0.0;
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) {
+                        const double v = d.alpha * s_out[(rb + r) * (kCols + 1) + lane];
+                        if (rb + r < nr) C[(rb + r) * d.ldc] = d.beta != 0.0 ? fma(d.beta, c[r], v) : v;
                     }
-                    if (ea >= kOzNan || eb >= kOzNan) v = __longlong_as_double(0x7ff8000000000000LL);
-                    if (scaled) v *= d.alpha;
-                    if (d.beta != 0.0) v = fma(d.beta, C[gj], v);
-                    C[gj] = v;
                 }
             }
         }

@@ -75,3 +75,18 @@ def test_fp64_sweep_rows(nk, spacing):
     ref = psi1_direct(pop.k0, pop.g0, pop.w0, kk[i], kg[j])
     d = np.abs(L[np.ix_(i, j)] - ref)
     assert np.all(d <= np.where(np.abs(ref) > 100, 1e-12 * np.abs(ref), 1e-10)), d.max()
+
+
+def test_subnormal_products():
+    """A Phi scaled by 2^-1015 takes the smaller outputs below the normal numbers: P and norm scale with it.  Subnormal
+    steps of 2^-1074 in a few hundred terms stay below 1e-12 of the largest sums (above 2^-1015)."""
+    from sgl_analytic_gb300._lib import SGL_FP64, Engine
+    g = _grid(331, 1203, 601, 257)
+    kk, kg = np.linspace(0, g["k_k_max"], g["nk_k"]), np.linspace(0, g["k_g_max"], g["nk_g"])
+    phi = np.exp(-0.5 * (0.05 * kk[:, None]) ** 2 - 0.5 * (0.05 * kg[None, :]) ** 2 - 0.01j * kk[:, None])
+    x = np.linspace(-0.2, 0.4, 101)
+    e = Engine(0)
+    P, m = e.invert_phi(phi, g, x, precision=SGL_FP64)
+    Q, n = e.invert_phi(phi * 2.0 ** -1015, g, x, precision=SGL_FP64)
+    assert abs(n["norm"] * 2.0 ** 1015 - m["norm"]) <= 1e-12 * abs(m["norm"])
+    assert np.max(np.abs(Q - P)) <= 2e-12 * np.max(np.abs(P))
