@@ -344,7 +344,7 @@ sgl_status xi_eval(sgl_ctx* ctx, int precision, const double* d_kk, const double
         CKLAUNCH();
         {
             Timed t(ctx, "xi_fused", fl, 0.0);
-            launch_xi_fused(ctx->xid, d_pp, d_pp + (ng + 1), d_jt, d_pre, cta_prefix[ng], d_pre + 2 * (ng + 1), Epk, J,
+            launch_xi_fused(ctx->xid, d_pp, d_pp + (2 * ng + 1), d_jt, d_pre, cta_prefix[ng], d_pre + 2 * (ng + 1), Epk, J,
                             d_Vf, d_kres, d_hq, nk, nkg, part, err, d_re, d_im, st);
         }
         CKLAUNCH();
@@ -901,13 +901,13 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
     struct GPlan {
         std::vector<int> keep, order, pg, qg, qs, qpos, qord, qseg;
         int nP = 0, q0 = 0, qseg0 = 0, p0 = 0;
-        long long ent0 = 0, rowel0 = 0, row0 = 0, u0 = 0, w0 = 0, um0 = 0;
+        long long ent0 = 0, rowel0 = 0, rowf0 = 0, row0 = 0, u0 = 0, w0 = 0, um0 = 0;
     };
     std::vector<GPlan> plan(n_groups);
     std::vector<int> g_m, g_r, g_nP, idx_p, p_ptr{0}, ent_qg, g_nQ, idx_q;
-    std::vector<long long> g_p_off, g_ent_off, g_row_off, p_prefix{0}, rowel_off, g_q_off, g_u_off;
+    std::vector<long long> g_p_off, g_ent_off, g_row_off, p_prefix{0}, rowel_off, rowf_off, g_q_off, g_u_off;
     std::vector<int> kept;                      // groups with rows left after pruning
-    long long ent_total = 0, row_total = 0, rowel_total = 0, u_total = 0, w0_total = 0, um_total[3] = {0, 0, 0};
+    long long ent_total = 0, row_total = 0, rowel_total = 0, rowf_total = 0, u_total = 0, w0_total = 0, um_total[3] = {0, 0, 0};
     // per-group index work in parallel (entry order by p, unique q), then the keep lists from the
     // norms, then the serial offsets and the parallel concatenation in group order
     std::atomic<int> bad_index{0};
@@ -970,7 +970,7 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
         g_nQ.push_back((int)P.qs.size());
         q_total += (long long)P.qs.size();
         if (coherent) qseg_total += (long long)P.qs.size() + 1;
-        P.ent0 = ent_total; P.rowel0 = rowel_total; P.row0 = row_total; P.u0 = u_total;
+        P.ent0 = ent_total; P.rowel0 = rowel_total; P.rowf0 = rowf_total; P.row0 = row_total; P.u0 = u_total;
         P.w0 = w0_total; P.um0 = um_total[mg];
         if (mg == 0) { w0_total += (long long)R * X.n_kmc; X.R0 += R; }
         um_total[mg] += (long long)R * X.n_gmc;
@@ -981,10 +981,12 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
         g_ent_off.push_back(ent_total);
         g_row_off.push_back(row_total);
         rowel_off.push_back(rowel_total);
+        rowf_off.push_back(rowf_total);
         p_prefix.push_back(p_prefix.back() + P.nP);
         ent_total += nidx[g];
         row_total += R;
         rowel_total += (long long)R * nidx[g];
+        rowf_total += (long long)xi_pad(R) * nidx[g];
         X.m.push_back(mg); X.r.push_back(R); X.nP.push_back(P.nP);
         kept.push_back(g);
     }
@@ -1045,6 +1047,7 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
                 XiPrepRow k{};
                 k.src = row_off[g] + (long long)P.keep[rr] * w;
                 k.dst = P.rowel0 + rr;
+                k.dstf = P.rowf0;
                 k.ent0 = P.ent0;
                 k.u_off = ubase[m[g]] + P.um0 + (long long)rr * X.n_gmc;
                 k.u0_off = P.u0 + (long long)rr * P.qs.size();
@@ -1066,7 +1069,7 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
             DBUF(d_idxq0, int, "xi_idxq", idx_q.size());
             DBUF(d_kmc0, double, "xi_kmc", X.n_kmc);
             DBUF(d_rows0, double, "xi_rows", rowel_total);
-            DBUF(d_rowsf0, float, "xi_rows_f", rowel_total + kXiTailPad);
+            DBUF(d_rowsf0, float, "xi_rows_f", rowf_total);
             DBUF(d_res0, double, "xi_res", row_total);
             DBUF(d_sum0, double, "xi_sum", row_total);
             DBUF(d_sig0, double, "xi_prep_sig", std::max<long long>(1, row_total));
@@ -1112,7 +1115,7 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
     if (!dev_filled) {
     // the transposed rows (FP64 and FP32 copies) are written straight into pinned memory
     CKS(sync_stream(ctx));
-    char* bp = big_pinned(ctx, (size_t)rowel_total * 12 + 256);
+    char* bp = big_pinned(ctx, (size_t)rowel_total * 8 + (size_t)rowf_total * 4 + 256);
     if (!bp) return fail(ctx, SGL_ERR_CUDA, "pinned host allocation failed (xi rows)");
     rows_t_p = (double*)bp;
     rows_tf_p = (float*)(bp + ((size_t)rowel_total * 8 + 255) / 256 * 256);
@@ -1125,7 +1128,8 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
         if (P.keep.empty()) return;
         const int R = (int)P.keep.size(), mg = m[g], w = nidx[g] + 1, ne = nidx[g];
         double* rt = rows_t_p + P.rowel0;
-        float* rtf = rows_tf_p + P.rowel0;
+        float* rtf = rows_tf_p + P.rowf0;
+        const int Rf = xi_pad(R);
         // rows_t[i][rr] = row_rr[order[i]], in blocks of entries so the strided writes stay in cache
         for (int i0 = 0; i0 < ne; i0 += 128) {
             const int i1 = std::min(ne, i0 + 128);
@@ -1134,9 +1138,10 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
                 for (int i = i0; i < i1; ++i) {
                     const double v = row[P.order[i]];
                     rt[(long long)i * R + rr] = v;
-                    rtf[(long long)i * R + rr] = (float)v;
+                    rtf[(long long)i * Rf + rr] = (float)v;
                 }
             }
+            for (int i = i0; i < i1; ++i) std::fill(rtf + (long long)i * Rf + R, rtf + (long long)(i + 1) * Rf, 0.f);
         }
         // one pass per kept row for its sums and the 1-D reach / compensation stacks (the same
         // per-output summation order as separate passes)
@@ -1204,10 +1209,10 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
         DBUF(d_gr, int, "xi_gr", X.n_groups);
         DBUF(d_gnP, int, "xi_gnP", X.n_groups);
         DBUF(d_goff, long long, "xi_goff", 3 * X.n_groups);
-        DBUF(d_pp, long long, "xi_pprefix", 2 * X.n_groups + 1);
+        DBUF(d_pp, long long, "xi_pprefix", 3 * X.n_groups + 1);
         DBUF(d_idxp, int, "xi_idxp", idx_p.size());
         DBUF(d_pptr, int, "xi_pptr", p_ptr.size());
-        DBUF(d_qg, int, "xi_entq", ent_qg.size() + kXiTailPad);
+        DBUF(d_qg, int, "xi_entq", ent_qg.size());
         DBUF(d_rows, double, "xi_rows", rowel_total);
         DBUF(d_res, double, "xi_res", res.size());
         DBUF(d_sum, double, "xi_sum", sum_rows.size());
@@ -1217,6 +1222,7 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
         goff.insert(goff.end(), g_row_off.begin(), g_row_off.end());
         std::vector<long long> pp = p_prefix;      // n_groups + 1
         pp.insert(pp.end(), rowel_off.begin(), rowel_off.end());
+        pp.insert(pp.end(), rowf_off.begin(), rowf_off.end());
         CKS(upload(ctx, d_gm, g_m.data(), g_m.size()));
         CKS(upload(ctx, d_gr, g_r.data(), g_r.size()));
         CKS(upload(ctx, d_gnP, g_nP.data(), g_nP.size()));
@@ -1237,9 +1243,9 @@ sgl_status sgl_lam_set_xi(sgl_ctx* ctx, int n_groups, const int32_t* m, const in
         D.g_p_off = d_goff; D.g_ent_off = d_goff + X.n_groups; D.g_row_off = d_goff + 2 * X.n_groups;
         D.idx_p = d_idxp; D.p_ptr = d_pptr; D.ent_qg = d_qg; D.rows = d_rows; D.res = d_res; D.sum_rows = d_sum;
         {
-            DBUF(d_rowsf, float, "xi_rows_f", rowel_total + kXiTailPad);
+            DBUF(d_rowsf, float, "xi_rows_f", rowf_total);
             if (rowel_total > 0 && !dev_filled)
-                CK(cudaMemcpyAsync(d_rowsf, rows_tf_p, (size_t)rowel_total * 4, cudaMemcpyHostToDevice, ctx->stream));
+                CK(cudaMemcpyAsync(d_rowsf, rows_tf_p, (size_t)rowf_total * 4, cudaMemcpyHostToDevice, ctx->stream));
             DBUF(d_gnQ, int, "xi_gnQ", g_nQ.size());
             DBUF(d_qoff, long long, "xi_qoff", g_q_off.size());
             DBUF(d_uoff, long long, "xi_uoff", g_u_off.size());

@@ -58,7 +58,7 @@ struct XiDevice {
     const int* p_ptr = nullptr;        // CSR over local p: entries [p_ptr[p], p_ptr[p+1]) (group relative)
     const int* ent_qg = nullptr;       // global gamma-centre index of each entry
     const double* rows = nullptr;      // rows: entry-major per group: rows[(ent_off + e) * r + rr]
-    const float* rows_f = nullptr;     // float copy of rows (mixed path)
+    const float* rows_f = nullptr;     // float copy of rows (mixed path), an entry's rows padded to xi_pad(r) with zeros
     int r_max = 0;                     // largest group row count
     const int* g_nQ = nullptr;         // unique gamma cells per group
     const long long* g_q_off = nullptr;   // into idx_q
@@ -97,11 +97,11 @@ void launch_xi_V_mixed(const XiDevice& x, const double* J0m1, int nkg, float* Vf
 // fused mixed gauss Psi_2 (tcgen05; xi_fused.cu): T built in shared memory, contracted with the
 // packed E in TMEM, squared and summed over rows in the epilogue
 int xi_fused_jt(int r);
-constexpr int kXiTailPad = 16;     // elements after rows_f and ent_qg: room for 16-byte-aligned bulk copies
+__host__ __device__ constexpr int xi_pad(int r) { return (r + 3) & ~3; }      // rows of an entry in rows_f: 16-byte loads
 bool xi_fused_fits(int r_max, int nk, int n_gmc);
 void launch_xi_E_pack(const XiDevice& x, const double* kk, int nk, const long long* pp_prefix, long long total_pp,
                       const long long* p_prefix, const long long* e_off, float* Epk, cudaStream_t st);
-void launch_xi_fused(const XiDevice& x, const long long* p_prefix, const long long* rowel_off, const int* jt,
+void launch_xi_fused(const XiDevice& x, const long long* p_prefix, const long long* rowf_off, const int* jt,
                      const long long* cta_prefix, long long ctas, const long long* e_off, const float* Epk,
                      const float* J, const float* Vf, const float2* kresT, const float2* hq, int nk, int nkg,
                      float2* part, int* err, double* out_re, double* out_im, cudaStream_t st);
@@ -264,6 +264,7 @@ void launch_adamw(long long n, float* w, const float* g, float* m, float* v, flo
 struct XiPrepRow {                 // one kept row
     long long src;                 // first element of the raw row in the caller's rows
     long long dst;                 // rows_t offset of entry 0 of its group, + rr
+    long long dstf;                // offset of the group in the padded FP32 copy
     long long ent0;                // group's first entry (inverse / q / p orders)
     long long u_off, u0_off, w0_off;   // row starts in U[m], U0, W0
     int ne, R, row, m;             // entries, kept rows of the group, global kept-row index, harmonic

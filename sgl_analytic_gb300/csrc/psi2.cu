@@ -76,7 +76,7 @@ k_xi_stageA(XiDevice x, const long long* __restrict__ p_prefix, const long long*
     const TT* Jm = J + (long long)m * x.n_gmc * nkg;
     TT* Tg = T + T_off[g] + (long long)p * r * nkg;
     const double* rows = x.rows + rowel_off[g];
-    const float* rows_f = x.rows_f ? x.rows_f + rowel_off[g] : nullptr;
+    const float* rows_f = x.rows_f ? x.rows_f + rowel_off[x.n_groups + g] : nullptr;
     constexpr int kMaxOut = 24;                               // outputs per thread (r * nkg <= 256 * 24)
     TT acc[kMaxOut];
 #pragma unroll
@@ -88,7 +88,7 @@ k_xi_stageA(XiDevice x, const long long* __restrict__ p_prefix, const long long*
         for (int t = threadIdx.x; t < cnt * r; t += blockDim.x) {
             const int e = t / r, rr = t % r;
             const long long el = (long long)(eb + e) - ent0;
-            s_rows[e * r + rr] = (sizeof(TT) == 4 && rows_f) ? (TT)rows_f[el * r + rr] : (TT)rows[el * r + rr];
+            s_rows[e * r + rr] = (sizeof(TT) == 4 && rows_f) ? (TT)rows_f[el * xi_pad(r) + rr] : (TT)rows[el * r + rr];
         }
         for (int t = threadIdx.x; t < cnt * nkg; t += blockDim.x) {
             const int e = t / nkg, j = t % nkg;
@@ -140,7 +140,7 @@ k_xi_stageA_generic(XiDevice x, const long long* __restrict__ p_prefix, const lo
 
 void launch_xi_stageA(int precision, const XiDevice& x, const long long* d_p_prefix, int total_p, const long long* T_off,
                       const void* J, int nkg, void* T, cudaStream_t st) {
-    // rowel_off is stored right after p_prefix in the same device block (see capi)
+    // rowel_off, then the offsets into rows_f, are stored right after p_prefix in the same device block
     const long long* rowel_off = d_p_prefix + (x.n_groups + 1);
     const int rmax = x.r_max;
     if (nkg > 128 || (long long)rmax * nkg > 256LL * 24) {
@@ -199,7 +199,7 @@ k_xi_stageA_pack(XiDevice x, const long long* __restrict__ p_prefix, const long 
     const int M = r * nkg;
     const int nrb = rp / 4, njb = nkp / 4, ntask = nrb * njb;
     const long long gp0 = p_prefix[g], ent0 = x.g_ent_off[g];
-    const float* rowsg = x.rows_f + rowel_off[g];
+    const float* rowsg = x.rows_f + rowel_off[x.n_groups + g];
     const float* Jm = J + (long long)m * x.n_gmc * nkg;
     const int tid = threadIdx.x;
     for (int pp = 0; pp < 4; ++pp) {
@@ -221,7 +221,7 @@ k_xi_stageA_pack(XiDevice x, const long long* __restrict__ p_prefix, const long 
             __syncthreads();
             for (int t = tid; t < kSAEnt * rp; t += kSAThreads) {
                 const int e = t / rp, rr = t % rp;
-                s_rows[e * rp + rr] = (e < cnt && rr < r) ? rowsg[((long long)(eb + e) - ent0) * r + rr] : 0.f;
+                s_rows[e * rp + rr] = (e < cnt && rr < r) ? rowsg[((long long)(eb + e) - ent0) * rp + rr] : 0.f;
             }
             for (int t = tid; t < kSAEnt * nkp; t += kSAThreads) {
                 const int e = t / nkp, j = t % nkp;
@@ -312,7 +312,7 @@ k_xi_stageA_pack_reg(XiDevice x, const long long* __restrict__ p_prefix, const l
     const int M = r * nkg;
     const int njb = nkp / 4, ntask = (rp / 4) * njb;
     const long long gp0 = p_prefix[g], ent0 = x.g_ent_off[g];
-    const float* rowsg = x.rows_f + rowel_off[g];
+    const float* rowsg = x.rows_f + rowel_off[x.n_groups + g];
     const float* Jm = J + (long long)m * x.n_gmc * nkg;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool has_task = tid < ntask;
@@ -332,7 +332,7 @@ k_xi_stageA_pack_reg(XiDevice x, const long long* __restrict__ p_prefix, const l
         __syncthreads();
         // one round trip for the whole batch: every copy is issued before any is waited on
         for (int e = warp; e < cnt; e += kSAThreads / 32) {
-            const float* src = rowsg + ((long long)(eb + e) - ent0) * r;
+            const float* src = rowsg + ((long long)(eb + e) - ent0) * rp;
             for (int rr = lane; rr < rp; rr += 32) {
                 if (rr < r) cp_async4(s_rows + e * rpm + rr, src + rr);
                 else s_rows[e * rpm + rr] = 0.f;

@@ -11,18 +11,24 @@
 // of the epilogue holds every row rr of its (n, j) and sums over them without communication.  T and
 // G never reach global memory: the unfused form writes and re-reads about 2 GB of them per PDF.
 //
+// Columns c = jl xi_pad(r) + rr: rows padded to a multiple of four, so that four rows of an entry are one 16-byte load.
+//
 // Pipeline (kXfStages shared-memory stages of 64 KB: E 4 x 8 KB [part][cos | sin], T 2 x 16 KB [part]):
-//   12 producer warps build the T tile of a 16-p K block from the CSR entries: 3 warps per 4-p block,
-//                     lanes over (column half, row) tasks; each block's entries (rows and gamma-cell
-//                     indices) stream through its own two shared-memory chunk buffers by bulk copy,
-//                     J_m of the CTA's columns is staged once; T is split into TF32 hi + lo and
-//                     stored in the canonical K-major layout; fence.proxy.async, one arrival per warp;
+//   12 producer warps build the T tiles of 16-p K blocks from the CSR entries, each warp 4-p blocks of its own
+//                     (every twelfth), eight lanes per p: lane = (p, row quads, column half) with the sums of up to
+//                     12 rows x 4 columns in registers.  Rows and gamma-cell indices come straight from global memory
+//                     (L2), four entries' loads in flight per lane; J_m of the CTA's columns is staged once; the
+//                     sums are transposed among the four p's lanes, split into TF32 hi + lo and stored in the
+//                     canonical K-major layout; fence.proxy.async, one arrival per block;
 //   1 copy thread     brings the packed E block (both parts, both halves) with one bulk copy;
 //   1 MMA thread      issues A0 B0 + A0 B1 + A1 B0 (TF32 hi/lo, ~2^-21 per product) into the cos and
-//                     sin accumulators (TMEM columns 0 and 256) and commits each stage to its "empty"
+//                     sin accumulators (TMEM columns 0 and 256) and commits each K block to its "empty"
 //                     barrier.
+// What bounds it: the producers, waiting for L2 (1.5-2k cycles per batch of loads, three warps per scheduler).  A CTA of
+// the reference's z_s = 1 groups (35 rows, 254 p, 3,928 entries) takes 109k cycles: prologue 4k, tiles 95k (the MMAs 25k,
+// hidden), last products 5k, squares 5k.  One launch: 1.55 -> 1.36 ms (three warps per 4-p block with a group barrier and
+// a bulk copy per chunk of entries, squares with a test per column: 147k cycles a CTA).
 // The summation order of T over entries and of the squares over rr is that of the unfused kernels.
-// The epilogue's correction terms are staged by the producers in the freed chunk buffers.
 // Every wait is bounded; a wait that runs out sets *err and the CTA skips to its TMEM release.
 #include "kernels.cuh"
 #include "tcgen05.cuh"
@@ -33,28 +39,22 @@ constexpr int kXfStages = 2;
 constexpr int kXfABytes = 4 * 8192;                  // E: [part][cos | sin] x 128 lanes x 16 p
 constexpr int kXfBPart = 16384;                      // T: 256 columns x 16 p, per part
 constexpr int kXfStageBytes = kXfABytes + 2 * kXfBPart;
-constexpr int kXfRMax = 48;                          // rows per group (2 r tasks <= producer threads)
-constexpr int kXfGroupWarps = 3;                     // producer warps per 4-p block
-constexpr int kXfProdWarps = 4 * kXfGroupWarps;
+constexpr int kXfRMax = 48;                          // rows per group: 3 row quads for each of 4 lanes
+constexpr int kXfProdWarps = 12;
 constexpr int kXfProd = kXfProdWarps * 32;
 constexpr int kXfThreads = kXfProd + 64;             // + copy warp + MMA warp
+constexpr int kXfParts = kXfProdWarps / 4;           // column parts of the epilogue
 constexpr int kXfJt = 8;                             // k_gamma columns per CTA at most
-constexpr int kXfChunk = 64;                         // entries per chunk of one warp group, at most
-constexpr int kXfRowsCap = 64 * 36;                  // row values per chunk buffer: 64 entries of <= 36 rows,
-                                                     // fewer entries per chunk for longer groups
+constexpr int kXfBlocks = 4;                         // 4-p blocks of a K block
+// A parity tells a barrier's phase from its neighbours only, and a producer warp's blocks are kXfProdWarps / kXfBlocks
+// = 3 K blocks apart: with a barrier per stage it would meet one that is two phases behind and pass.  One per K block
+// modulo 8: a waiter for kb is less than 8 K blocks from any K block that shares it.
+constexpr int kXfEmpty = 8;
+static_assert(kXfProdWarps / kXfBlocks + 2 * kXfStages < kXfEmpty, "waits for a K block's barrier are unambiguous");
+constexpr int kXfBatch = 4;                          // entries whose loads are in flight per lane
 constexpr int kXfSmemStages = kXfStages * kXfStageBytes;
-constexpr int kXfRowsBuf = kXfRowsCap * 4 + 64;      // + room for the aligned superset
-constexpr int kXfQBuf = kXfChunk * 4 + 64;
-constexpr int kXfBlocks = 4;                          // producer warp groups, one per 4-p block of a K block
-constexpr int kXfChunkBytes = kXfBlocks * 2 * (kXfRowsBuf + kXfQBuf);
-constexpr int kXfSmemFixed = kXfSmemStages + kXfChunkBytes;
-static_assert(2 * kXfRMax <= 32 * kXfGroupWarps, "one (row, column half) task per producer lane");
-static_assert(kXfRMax * 128 * 8 + kXfRMax * kXfJt * 8 <= kXfChunkBytes, "epilogue tables fit the chunk buffers");
-static_assert(kXfRowsCap / kXfRMax >= 4, "a chunk holds a few entries of the longest group");
-
-// entries per chunk for a group of r rows: the chunk's rows fill at most kXfRowsCap values
-__host__ __device__ constexpr int xf_chunk_entries(int r) { return r * kXfChunk <= kXfRowsCap ? kXfChunk : kXfRowsCap / r; }
-
+constexpr int kXfTabBytes = kXfRMax * 128 * 8 + kXfRMax * kXfJt * 8;     // the epilogue's correction terms
+constexpr int kXfSmemFixed = kXfSmemStages + kXfTabBytes;
 
 __device__ __forceinline__ int xf_find(const long long* prefix, int ng, long long v) {
     int lo = 0, hi = ng - 1;                          // largest g with prefix[g] <= v
@@ -71,10 +71,23 @@ __device__ __forceinline__ float xf_add_ff(float b, float2 hl) {   // round(b + 
     return s + (err + hl.y);
 }
 
-int xi_fused_jt(int r) { return r <= 0 ? 0 : std::min(kXfJt, 256 / r); }
+// four columns of a warp's lanes, asynchronous; xf_ld_wait names the registers, so that nothing reads them before it
+__device__ __forceinline__ void xf_ld4(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr));
+}
+__device__ __forceinline__ void xf_ld_wait(uint32_t* v) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
+                   "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23])
+                 :: "memory");
+}
 
-// stages, entry chunks, J_m columns, then the mbarriers, the TMEM address and the failure flag
-size_t xi_fused_smem(int n_gmc) { return (size_t)kXfSmemFixed + (size_t)n_gmc * kXfJt * 4 + 8 * (2 * kXfStages + 1 + 2 * kXfBlocks) + 32; }
+int xi_fused_jt(int r) { return r <= 0 ? 0 : std::min(kXfJt, 256 / xi_pad(r)); }
+
+// stages, correction terms, J_m columns, then the mbarriers, the TMEM address and the failure flag
+size_t xi_fused_smem(int n_gmc) { return (size_t)kXfSmemFixed + (size_t)n_gmc * kXfJt * 4 + 8 * (kXfStages + kXfEmpty + 1) + 32; }
 
 bool xi_fused_fits(int r_max, int nk, int n_gmc) {
     return nk >= 1 && nk <= 128 && r_max >= 1 && r_max <= kXfRMax && xi_fused_smem(n_gmc) <= 227 * 1024;
@@ -112,7 +125,7 @@ k_xi_E_pack(XiDevice x, const double* __restrict__ kk, int nk, const long long* 
 struct XiFusedArgs {
     XiDevice x;
     const long long* p_prefix;      // [n_groups + 1] global index of each group's first p
-    const long long* rowel_off;     // [n_groups] float offset of each group's rows
+    const long long* rowf_off;      // [n_groups] float offset of each group's padded rows
     const int* jt;                  // [n_groups] k_gamma columns per CTA
     const long long* cta_prefix;    // [n_groups + 1]
     const long long* e_off;         // [n_groups] packed E offsets (floats)
@@ -126,9 +139,44 @@ struct XiFusedArgs {
     int* err;
 };
 
-// one entry chunk of a warp group: entries [ea, eb) of its 4-p block in K block kb, at most
-// xf_chunk_entries(r)
-struct XfChunk { int kb, ea, eb; };
+// ( sum_rr (a^2 - b^2), sum_rr a b ) of one k_gamma column, rows in order: cos sums at TMEM column col, sin sums 256 on.
+// Twelve rows' loads under one wait and the harmonic's form fixed at compile time: with a test per column this took 27k
+// cycles of a CTA (5k now).
+template <int M>
+__device__ __forceinline__ float2 xf_square(uint32_t col, int nq, int r, bool any, const float2* __restrict__ cor,
+                                            const float2* __restrict__ kres) {
+    float gre = 0.f, gim = 0.f;
+    for (int Q0 = 0; Q0 < nq; Q0 += 3) {
+        uint32_t v[3][8];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if (any && Q0 + i < nq) {
+                xf_ld4(col + (uint32_t)(4 * (Q0 + i)), v[i]);
+                xf_ld4(col + 256u + (uint32_t)(4 * (Q0 + i)), v[i] + 4);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[i][k] = 0u;
+            }
+        if (any) xf_ld_wait(&v[0][0]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int rr = 4 * (Q0 + i) + k;
+                if (rr >= r) break;                          // (the padded rows)
+                float av = __uint_as_float(v[i][k]), bv = __uint_as_float(v[i][4 + k]);
+                if (M == 0) {
+                    av += cor[rr * kXfJt].x;
+                    bv = xf_add_ff(bv, kres[rr * 128]);
+                } else if (M == 1) {
+                    av = xf_add_ff(av, cor[rr * kXfJt]);
+                }
+                gre = fmaf(av, av, fmaf(-bv, bv, gre));
+                gim = fmaf(av, bv, gim);
+            }
+    }
+    return make_float2(gre, gim);
+}
 
 __global__ void __launch_bounds__(kXfThreads, 1)
 k_xi_fused(XiFusedArgs a) {
@@ -140,32 +188,30 @@ k_xi_fused(XiFusedArgs a) {
     const int jt = a.jt[g];
     const int j0 = (int)(cta - a.cta_prefix[g]) * jt;
     const int r = x.g_r[g], m = x.g_m[g], nP = x.g_nP[g];
-    const int N = ((jt * r + 15) / 16) * 16;            // MMA N (<= 256)
+    const int r4 = xi_pad(r), nq = r4 / 4;
+    const int N = ((jt * r4 + 15) / 16) * 16;           // MMA N (<= 256)
     const int nkb = (nP + 15) / 16;
     const int nk = a.nk, nkg = a.nkg, n_gmc = x.n_gmc;
     float* s_J = (float*)(xsm + kXfSmemFixed);                           // [n_gmc][8]
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(xsm);
     const uint32_t boff = kXfSmemFixed + n_gmc * kXfJt * 4;
-    const uint32_t bar = sbase + boff;                   // full[S], empty[S], done, chunk[groups][2]
-    constexpr int kNBar = 2 * kXfStages + 1 + 2 * kXfBlocks;
+    const uint32_t bar = sbase + boff;                   // full[S], empty[kXfEmpty], done
+    constexpr int kNBar = kXfStages + kXfEmpty + 1;
     const uint32_t tslot = bar + 8 * kNBar;
     volatile int* s_fail = (volatile int*)(xsm + boff + 8 * kNBar + 8);
     auto full = [&](int s) { return bar + 8 * s; };
-    auto empty = [&](int s) { return bar + 8 * (kXfStages + s); };
-    const uint32_t done = bar + 8 * (2 * kXfStages);
-    auto cbar = [&](int pr, int b) { return bar + 8 * (2 * kXfStages + 1 + 2 * pr + b); };
+    auto empty = [&](int kb) { return bar + 8 * (kXfStages + kb % kXfEmpty); };
+    auto wait_consumed = [&](int kb) { return mbar_wait_sleep(empty(kb), (uint32_t)((kb / kXfEmpty) & 1)); };
+    const uint32_t done = bar + 8 * (kXfStages + kXfEmpty);
 
     if (warp == kXfProdWarps + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(tslot), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int s = 0; s < kXfStages; ++s) {
-            mbar_init(full(s), kXfProdWarps + 1);
-            mbar_init(empty(s), 1);
-        }
+        for (int s = 0; s < kXfStages; ++s) mbar_init(full(s), kXfBlocks + 1);
+        for (int e = 0; e < kXfEmpty; ++e) mbar_init(empty(e), 1);
         mbar_init(done, 1);
-        for (int b = 0; b < 2 * kXfBlocks; ++b) mbar_init(cbar(b >> 1, b & 1), 1);
         *s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -182,168 +228,100 @@ k_xi_fused(XiFusedArgs a) {
     const uint32_t tmem = *(volatile uint32_t*)(xsm + boff + 8 * kNBar);
 
     if (warp < kXfProdWarps && nkb > 0) {
-        // ---- T producers: warp group pb (kXfGroupWarps warps) owns p = 16 kb + 4 pb .. + 3 of every
-        // K block; its lanes take the tasks (column half jh, row rr), t = jh r + rr < 2 r.  The group
-        // streams its own entries (CSR by p: one contiguous run per K block) through its own two chunk
-        // buffers: lane 0 of the group's first warp brings a chunk's rows and gamma-cell indices with
-        // two bulk copies of their 16-byte-aligned supersets, one chunk ahead of the one being summed.
-        // The groups run independently; the full barrier of a stage collects one arrival per warp.
-        const long long gp0 = a.p_prefix[g], ent0 = x.g_ent_off[g];
-        const float* rowsg = x.rows_f + a.rowel_off[g];
-        const int* pptr = x.p_ptr + gp0;
-        const int pb = warp / kXfGroupWarps, sub = warp % kXfGroupWarps;
-        const int t = sub * 32 + lane;
-        const bool active = t < 2 * r;
-        const int jh = active ? t / r : 0, rr = active ? t - jh * r : 0;
-        const bool issuer = sub == 0 && lane == 0;
-        float* const rbuf0 = (float*)(xsm + kXfSmemStages + (pb * 2) * kXfRowsBuf);
-        int* const qbuf0 = (int*)(xsm + kXfSmemStages + 2 * kXfBlocks * kXfRowsBuf + (pb * 2) * kXfQBuf);
-        auto lo_of = [&](int kb) { return pptr[min(16 * kb + 4 * pb, nP)]; };
-        auto hi_of = [&](int kb) { return pptr[min(16 * kb + 4 * pb + 4, nP)]; };
-        auto rows_at = [&](int e) { return rowsg + (long long)(e - ent0) * r; };
-        auto issue = [&](XfChunk c, int buf) {          // issuer lane only
-            const uint32_t cb = cbar(pb, buf);
-            if (c.eb == c.ea) { mbar_arrive(cb); return; }
-            const uintptr_t r0 = (uintptr_t)rows_at(c.ea), r1 = (uintptr_t)rows_at(c.eb);
-            const uintptr_t q0 = (uintptr_t)(x.ent_qg + c.ea), q1 = (uintptr_t)(x.ent_qg + c.eb);
-            const uintptr_t r0a = r0 & ~(uintptr_t)15, q0a = q0 & ~(uintptr_t)15;
-            const uint32_t rb = (uint32_t)(((r1 + 15) & ~(uintptr_t)15) - r0a);
-            const uint32_t qb = (uint32_t)(((q1 + 15) & ~(uintptr_t)15) - q0a);
-            mbar_expect_tx(cb, rb + qb);
-            bulk_g2s((uint32_t)__cvta_generic_to_shared(rbuf0) + buf * kXfRowsBuf, (const void*)r0a, rb, cb);
-            bulk_g2s((uint32_t)__cvta_generic_to_shared(qbuf0) + buf * kXfQBuf, (const void*)q0a, qb, cb);
-        };
-        const int chunk = xf_chunk_entries(r);
-        XfChunk cur{0, lo_of(0), 0};
-        int cur_hi = hi_of(0);
-        cur.eb = min(cur.ea + chunk, cur_hi);
-        if (issuer) issue(cur, 0);
-        int ci = 0, issued = 0;                         // chunk counters: buffer ci & 1, parity (ci >> 1) & 1
-        float acc[4][4];                                // [p of the block][column of the half]
+        // ---- T producers.  Lane (u, rg, jh): p = 4 b + u of block b, row quads rg, rg + 4, rg + 8, columns 4 jh .. + 3;
+        // an entry's sums run over the entries in order
+        const int u = lane & 3, rg = (lane >> 2) & 3, jh = lane >> 4;
+        const int* pptr = x.p_ptr + a.p_prefix[g];
+        const float4* rows4 = (const float4*)(x.rows_f + a.rowf_off[g]) + rg;
+        const long long ent0 = x.g_ent_off[g];
+        const float* sj = s_J + 4 * jh;
+        const int nslot = (nq + 3) / 4;                     // row quads of a lane (the last for some lanes only)
+        const int nblk = kXfBlocks * nkb;
+        int e0 = pptr[min(4 * warp + u, nP)], e1 = pptr[min(4 * warp + u + 1, nP)];
+        for (int b = warp; b < nblk; b += kXfProdWarps) {
+            const int n = e1 - e0, nmax = __reduce_max_sync(0xffffffffu, n);
+            const int* qg = x.ent_qg + e0;
+            const float4* rp = rows4 + ((long long)e0 - ent0) * nq;
+            const int bn = b + kXfProdWarps;                // the next block's bounds, while this one is summed
+            e0 = pptr[min(4 * bn + u, nP)];
+            e1 = pptr[min(4 * bn + u + 1, nP)];
+            float acc[3][4][4];                             // [row quad][row][column]
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+            for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int w = 0; w < 4; ++w) acc[u][w] = 0.f;
-        int pbnd[5];
+                for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int u = 0; u < 5; ++u) pbnd[u] = pptr[min(4 * pb + u, nP)];
-        bool failed = false;
-        while (cur.kb < nkb) {
-            // group barrier (the buffer of the previous chunk is free) that also ORs the warps'
-            // failure flags, so that they leave the loop together
-            int any_fail;
-            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
-                         "bar.red.or.pred q, %2, %3, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
-                         : "=r"(any_fail) : "r"((failed || *s_fail) ? 1 : 0), "r"(1 + pb), "r"(32 * kXfGroupWarps)
-                         : "memory");
-            if (any_fail) break;
-            XfChunk nxt;
-            int nxt_hi = cur_hi;
-            if (cur.eb < cur_hi) {
-                nxt.kb = cur.kb; nxt.ea = cur.eb;
-            } else {
-                nxt.kb = cur.kb + 1;
-                nxt.ea = nxt.kb < nkb ? lo_of(nxt.kb) : 0;
-                nxt_hi = nxt.kb < nkb ? hi_of(nxt.kb) : 0;
-            }
-            nxt.eb = nxt.kb < nkb ? min(nxt.ea + chunk, nxt_hi) : nxt.ea;
-            if (nxt.kb < nkb) {
-                if (issuer) issue(nxt, (ci + 1) & 1);
-                issued = ci + 1;
-            }
-            const int b = ci & 1;
-            if (!mbar_wait_sleep(cbar(pb, b), (uint32_t)((ci >> 1) & 1))) failed = true;
-            if (!failed && cur.eb > cur.ea && active) {
-                const int rlead = (int)(((uintptr_t)rows_at(cur.ea) & 15) >> 2);
-                const int qlead = (int)(((uintptr_t)(x.ent_qg + cur.ea) & 15) >> 2);
-                const float* sr = rbuf0 + b * (kXfRowsBuf / 4) + rlead + rr;
-                const int* sq = qbuf0 + b * (kXfQBuf / 4) + qlead;
-                const float* sj = s_J + 4 * jh;
+                    for (int w = 0; w < 4; ++w) acc[i][k][w] = 0.f;
+            for (int s0 = 0; s0 < nmax; s0 += kXfBatch) {
+                int q[kXfBatch];
+                float4 v[kXfBatch][3];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int e_lo = max(pbnd[u], cur.ea) - cur.ea, e_hi = min(pbnd[u + 1], cur.eb) - cur.ea;
-                    int e = e_lo;
-                    // four entries per step, their loads issued ahead of the FMAs (entry order kept)
-                    for (; e + 3 < e_hi; e += 4) {
-                        float4 jv[4];
-                        float v[4];
+                for (int k = 0; k < kXfBatch; ++k) {
+                    const bool in = s0 + k < n;
+                    q[k] = in ? __ldg(qg + s0 + k) * kXfJt : 0;
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            jv[k] = *(const float4*)(sj + sq[e + k] * kXfJt);
-                            v[k] = sr[(e + k) * r];
+                    for (int i = 0; i < 3; ++i)
+                        v[k][i] = in && rg + 4 * i < nq ? __ldg(rp + (s0 + k) * nq + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int k = 0; k < kXfBatch; ++k) {
+                    if (s0 + k >= nmax) break;
+                    const float4 j = *(const float4*)(sj + q[k]);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        if (i >= nslot) break;
+                        const float vv[4] = {v[k][i].x, v[k][i].y, v[k][i].z, v[k][i].w};
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) {
+                            acc[i][t][0] = fmaf(vv[t], j.x, acc[i][t][0]);
+                            acc[i][t][1] = fmaf(vv[t], j.y, acc[i][t][1]);
+                            acc[i][t][2] = fmaf(vv[t], j.z, acc[i][t][2]);
+                            acc[i][t][3] = fmaf(vv[t], j.w, acc[i][t][3]);
                         }
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            acc[u][0] = fmaf(v[k], jv[k].x, acc[u][0]);
-                            acc[u][1] = fmaf(v[k], jv[k].y, acc[u][1]);
-                            acc[u][2] = fmaf(v[k], jv[k].z, acc[u][2]);
-                            acc[u][3] = fmaf(v[k], jv[k].w, acc[u][3]);
-                        }
-                    }
-                    for (; e < e_hi; ++e) {
-                        const float4 j0 = *(const float4*)(sj + sq[e] * kXfJt);
-                        const float v0 = sr[e * r];
-                        acc[u][0] = fmaf(v0, j0.x, acc[u][0]);
-                        acc[u][1] = fmaf(v0, j0.y, acc[u][1]);
-                        acc[u][2] = fmaf(v0, j0.z, acc[u][2]);
-                        acc[u][3] = fmaf(v0, j0.w, acc[u][3]);
                     }
                 }
             }
-            if (nxt.kb != cur.kb) {
-                // the group's share of K block kb is complete: its stage must have been consumed by the
-                // MMAs of kb - S
-                const int kb = cur.kb, s = kb % kXfStages;
-                if (kb >= kXfStages && !mbar_wait_sleep(empty(s), (uint32_t)(((kb / kXfStages) - 1) & 1)))
-                    failed = true;                      // acted on at the next barrier
-                float* Bst = (float*)(xsm + s * kXfStageBytes + kXfABytes);
-                // column c = jl r + rr, K index 4 pb + u: one float4 (hi) + one (lo) per (row, column)
-                auto put = [&](const float (&av)[4][4], int rr) {
+            const int kb = b / kXfBlocks, pb = b % kXfBlocks, s = kb % kXfStages;
+            // its stage must have been consumed by the MMAs of kb - S
+            if (*s_fail || (kb >= kXfStages && !wait_consumed(kb - kXfStages))) {
+                *s_fail = 1;
+                break;
+            }
+            float* Bst = (float*)(xsm + s * kXfStageBytes + kXfABytes);
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        const int jl = 4 * jh + w;
-                        if (jl < jt) {
-                            const int c = jl * r + rr;
-                            float hv[4], lv[4];
+            for (int i = 0; i < 3; ++i) {
+                const int Q = rg + 4 * i;
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                hv[u] = tf32_rna(av[u][w]);
-                                lv[u] = tf32_rna(av[u][w] - hv[u]);
-                            }
-                            const int o = (c >> 3) * 128 + pb * 32 + (c & 7) * 4;
-                            *(float4*)(Bst + o) = make_float4(hv[0], hv[1], hv[2], hv[3]);
-                            *(float4*)(Bst + kXfBPart / 4 + o) = make_float4(lv[0], lv[1], lv[2], lv[3]);
-                        }
+                for (int w = 0; w < 4; ++w) {
+                    // transpose among the four p's lanes: lane u gets row 4 Q + u of the p's 0 .. 3
+                    float t0 = acc[i][0][w], t1 = acc[i][1][w], t2 = acc[i][2][w], t3 = acc[i][3][w];
+                    const float x0 = __shfl_xor_sync(0xffffffffu, u & 1 ? t0 : t1, 1);
+                    const float x1 = __shfl_xor_sync(0xffffffffu, u & 1 ? t2 : t3, 1);
+                    if (u & 1) { t0 = x0; t2 = x1; } else { t1 = x0; t3 = x1; }
+                    const float y0 = __shfl_xor_sync(0xffffffffu, u & 2 ? t0 : t2, 2);
+                    const float y1 = __shfl_xor_sync(0xffffffffu, u & 2 ? t1 : t3, 2);
+                    if (u & 2) { t0 = y0; t1 = y1; } else { t2 = y0; t3 = y1; }
+                    const int jl = 4 * jh + w;
+                    if (jl < jt && Q < nq) {
+                        // column c = jl r4 + 4 Q + u, K index 4 pb + (0 .. 3)
+                        const int cq = jl * nq + Q, o = (cq >> 1) * 128 + pb * 32 + (cq & 1) * 16 + u * 4;
+                        const float4 h = make_float4(tf32_rna(t0), tf32_rna(t1), tf32_rna(t2), tf32_rna(t3));
+                        *(float4*)(Bst + o) = h;
+                        *(float4*)(Bst + kXfBPart / 4 + o) =
+                            make_float4(tf32_rna(t0 - h.x), tf32_rna(t1 - h.y), tf32_rna(t2 - h.z), tf32_rna(t3 - h.w));
                     }
-                };
-                if (active) put(acc, rr);
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full(s));
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) acc[u][w] = 0.f;
-                if (nxt.kb < nkb) {
-#pragma unroll
-                    for (int u = 0; u < 5; ++u) pbnd[u] = pptr[min(16 * nxt.kb + 4 * pb + u, nP)];
                 }
             }
-            cur = nxt;
-            cur_hi = nxt_hi;
-            ++ci;
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full(s));
         }
-        // no bulk copy outlives the loop: the issuer waits (bounded) for any chunk it issued that was
-        // not consumed (only after a failure)
-        if (issuer)
-            for (int c = ci; c <= issued; ++c) mbar_wait_sleep(cbar(pb, c & 1), (uint32_t)((c >> 1) & 1));
-        if (failed) *s_fail = 1;
     } else if (warp == kXfProdWarps && lane == 0) {
         // ---- E: one bulk copy per K block (both parts, cos and sin halves)
         const float* Eg = a.Epk + a.e_off[g];
         for (int kb = 0; kb < nkb; ++kb) {
             const int s = kb % kXfStages;
-            if (kb >= kXfStages && (*s_fail || !mbar_wait_sleep(empty(s), (uint32_t)(((kb / kXfStages) - 1) & 1)))) {
+            if (kb >= kXfStages && (*s_fail || !wait_consumed(kb - kXfStages))) {
                 *s_fail = 1;
                 break;
             }
@@ -370,19 +348,17 @@ k_xi_fused(XiFusedArgs a) {
                         tc_mma(tmem + 256u * trig, tc_desc(a0 + (PA[t] * 2 + trig) * 8192 + o),
                                tc_desc(b0 + PB[t] * kXfBPart + o), idesc, (kb | ks | t) ? 1u : 0u);
             }
-            tc_commit(empty(s));
+            tc_commit(empty(kb));
         }
         tc_commit(done);
     }
 
-    // ---- epilogue.  Once every producer warp is done the chunk buffers are free: the producers
-    // stage there the square's correction terms for this CTA's rows and columns while the last
-    // MMAs run.
+    // ---- epilogue.  The producers that are done stage the square's correction terms for this CTA's rows and columns
+    // while the last tiles are built and the last MMAs run.
     const long long R0 = x.g_row_off[g];
     float2* s_kres = (float2*)(xsm + kXfSmemStages);                       // [r][128]  kk_n res (m = 0)
     float2* s_cor = (float2*)(xsm + kXfSmemStages + kXfRMax * 128 * 8);   // [r][8]    (V, 0) m = 0 / hq m = 1
     if (warp < kXfProdWarps) {
-        asm volatile("bar.sync 5, %0;" :: "r"(kXfProd) : "memory");
         for (int i = tid; i < r * 128; i += kXfProd) {
             const int rq = i >> 7, n = i & 127;
             s_kres[i] = (m == 0 && n < nk) ? a.kresT[(R0 + rq) * nk + n] : make_float2(0.f, 0.f);
@@ -404,45 +380,20 @@ k_xi_fused(XiFusedArgs a) {
     if (all_ok) {
         if (warp < kXfProdWarps) {
             // warp w reads TMEM lanes 32 (w % 4) .. + 31 (k_kappa index n) and the column part w / 4
-            // (of kXfGroupWarps) of the (jl, rr) pairs; the rows rr of one (n, j) are summed in registers
+            // (of kXfParts) of the (jl, rr) pairs; the rows rr of one (n, j) are summed in registers
             const int quad = warp & 3, part_ = warp >> 2;
             const int n = quad * 32 + lane;
-            const int jl_lo = (jt * part_) / kXfGroupWarps, jl_hi = (jt * (part_ + 1)) / kXfGroupWarps;
-            const int c_lo = jl_lo * r, c_hi = jl_hi * r;
-            int jl = jl_lo, rr = 0;
-            float gre = 0.f, gim = 0.f;
+            const int jl_lo = (jt * part_) / kXfParts, jl_hi = (jt * (part_ + 1)) / kXfParts;
             const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
-            for (int c0 = c_lo & ~15; c0 < c_hi; c0 += 16) {
-                float vc[16], vs[16];
-                if (nkb > 0) {
-                    tmem_ld16x2(lane_base + (uint32_t)c0, lane_base + 256u + (uint32_t)c0, vc, vs);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) { vc[q] = 0.f; vs[q] = 0.f; }
-                }
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    const int c = c0 + q;
-                    if (c < c_lo || c >= c_hi) continue;
-                    float av = vc[q], bv = vs[q];
-                    const float2 cor = s_cor[rr * kXfJt + jl];
-                    if (m == 0) {
-                        av += cor.x;
-                        bv = xf_add_ff(bv, s_kres[rr * 128 + n]);
-                    } else if (m == 1) {
-                        av = xf_add_ff(av, cor);
-                    }
-                    gre = fmaf(av, av, fmaf(-bv, bv, gre));
-                    gim = fmaf(av, bv, gim);
-                    if (++rr == r) {
-                        const int j = j0 + jl;
-                        if (n < nk && j < nkg) a.part[((long long)g * nkg + j) * nk + n] = make_float2(gre, gim);
-                        rr = 0;
-                        ++jl;
-                        gre = 0.f;
-                        gim = 0.f;
-                    }
-                }
+            for (int jl = jl_lo; jl < jl_hi; ++jl) {
+                const uint32_t col = lane_base + (uint32_t)(jl * r4);
+                const float2* cor = s_cor + jl;
+                float2 s = make_float2(0.f, 0.f);
+                if (m == 0) s = xf_square<0>(col, nq, r, nkb > 0, cor, s_kres + n);
+                else if (m == 1) s = xf_square<1>(col, nq, r, nkb > 0, cor, nullptr);
+                else s = xf_square<2>(col, nq, r, nkb > 0, cor, nullptr);
+                const int j = j0 + jl;
+                if (n < nk && j < nkg) a.part[((long long)g * nkg + j) * nk + n] = s;
             }
         }
     } else if (tid == 0) {
@@ -490,12 +441,12 @@ void launch_xi_E_pack(const XiDevice& x, const double* kk, int nk, const long lo
     SGL_COUNT(1);
 }
 
-void launch_xi_fused(const XiDevice& x, const long long* p_prefix, const long long* rowel_off, const int* jt,
+void launch_xi_fused(const XiDevice& x, const long long* p_prefix, const long long* rowf_off, const int* jt,
                      const long long* cta_prefix, long long ctas, const long long* e_off, const float* Epk,
                      const float* J, const float* Vf, const float2* kresT, const float2* hq, int nk, int nkg,
                      float2* part, int* err, double* out_re, double* out_im, cudaStream_t st) {
     if (ctas > 0) {
-        XiFusedArgs a{x, p_prefix, rowel_off, jt, cta_prefix, e_off, Epk, J, Vf, kresT, hq, nk, nkg, part, err};
+        XiFusedArgs a{x, p_prefix, rowf_off, jt, cta_prefix, e_off, Epk, J, Vf, kresT, hq, nk, nkg, part, err};
         const size_t sm = xi_fused_smem(x.n_gmc);
         cudaFuncSetAttribute(k_xi_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         k_xi_fused<<<(unsigned)ctas, kXfThreads, sm, st>>>(a);

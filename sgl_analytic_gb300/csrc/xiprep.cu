@@ -108,7 +108,7 @@ void launch_xi_stage_rows(const double* rows, long long n, double* dst, cudaStre
     SGL_COUNT(1);
 }
 
-// rows_t[i][rr] = row_rr[order[i]] (FP64 and FP32), one CTA per tile of kXiTransTile entries of a
+// rows_t[i][rr] = row_rr[order[i]] (FP64, and FP32 padded to xi_pad rows), one CTA per tile of kXiTransTile entries of a
 // group: the tile's rows_t region is contiguous, so the writes are coalesced; the gathers from the
 // group's rows hit L2.
 constexpr int kXiTransTile = 64;
@@ -124,12 +124,13 @@ k_xi_transpose(const double* __restrict__ rows, const XiPrepRow* __restrict__ kr
     for (int rr = threadIdx.x; rr < R; rr += blockDim.x) s_src[rr] = kr[tl.x + rr].src;
     for (int il = threadIdx.x; il < ni; il += blockDim.x) s_po[il] = pord[d0.ent0 + i0 + il];
     __syncthreads();
-    const long long base = d0.dst + (long long)i0 * R;
-    for (int t = threadIdx.x; t < ni * R; t += blockDim.x) {
-        const int il = t / R, rr = t - il * R;
-        const double v = rows[s_src[rr] + s_po[il]];
-        rt[base + t] = v;
-        rtf[base + t] = (float)v;
+    const int Rf = xi_pad(R);
+    const long long base = d0.dst + (long long)i0 * R, basef = d0.dstf + (long long)i0 * Rf;
+    for (int t = threadIdx.x; t < ni * Rf; t += blockDim.x) {
+        const int il = t / Rf, rr = t - il * Rf;
+        const double v = rr < R ? rows[s_src[rr] + s_po[il]] : 0.0;
+        if (rr < R) rt[base + il * R + rr] = v;
+        rtf[basef + t] = (float)v;
     }
 }
 
