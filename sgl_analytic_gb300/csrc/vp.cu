@@ -890,95 +890,108 @@ k_vp_chain_ff(VpDevice d, const float2* __restrict__ Kff, const double2* __restr
     }
 }
 
-// The same chain for few points (the k-reach probe lines): one CTA per point, one thread per state.
-// The per-state work (mat-vec over i in the same order, exp, sincos, normalisation) runs in
-// parallel; the two ordered sums (the projection's weighted mean, the final state sum) stay on
-// one thread in state order, and the maxima are order-free, so the results are those of
-// k_vp_chain.
-constexpr int kChSmallThreads = 64;
+// z and A_lin of a shell's pieces into the first one's place, in piece order
+__global__ void k_vp_sum_pieces(double2* __restrict__ zp, long long nz, double2* __restrict__ alin, long long na, int npieces) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nz + na) return;
+    double2* x = t < nz ? zp + t : alin + (t - nz);
+    const long long stride = t < nz ? nz : na;
+    double2 v = x[0];
+#pragma unroll 8
+    for (int pc = 1; pc < npieces; ++pc) {
+        const double2 a = x[pc * stride];
+        v.x += a.x; v.y += a.y;
+    }
+    x[0] = v;
+}
+
+// The same chain for few points (the k-reach probe lines): one CTA per point, two threads per state, one for the real
+// parts and one (in other warps) for the imaginary ones.  The per-state work (mat-vec over i in the same order, exp beside
+// sincos, normalisation) runs in parallel; the ordered sums (the projection's weighted means, the final state sums) stay on
+// one thread each in state order, and the maxima are order-free, so the results are those of k_vp_chain.  Bound by the
+// FP64 instructions of a shell in sequence (a warp's takes 64 cycles): 20 points, 24 shells, 26 pieces 0.63 -> 0.21 ms
+// (pieces summed, K fetched and both parts' products formed by the same 64 threads, in turn).
+constexpr int kChHalf = 64, kChSmallThreads = 2 * kChHalf;
 
 __global__ void __launch_bounds__(kChSmallThreads)
 k_vp_chain_small(VpDevice d, const double2* __restrict__ zp, const double2* __restrict__ alin, long long NP, int nq,
-                 int kb, double* __restrict__ out_re, double* __restrict__ out_im, int npieces) {
-    __shared__ double sK[kVpNS * kVpNS];
-    __shared__ double zr_s[kVpNS], zi_s[kVpNS], ar[kVpNS], ai[kVpNS];
-    __shared__ double red[kChSmallThreads];
-    __shared__ double s_mr, s_mi;
-    const int j = threadIdx.x;
+                 int kb, double* __restrict__ out_re, double* __restrict__ out_im) {
+    __shared__ __align__(16) double sK[2][kVpNS * kVpNS];
+    __shared__ double sw[kVpNS], z_s[2][kVpNS], al_s[2][kVpNS], g_s[2][kVpNS], n_s[2][kVpNS], mn[2], ex_s[kVpNS];
+    __shared__ double2 tr_s[kVpNS];
+    __shared__ double red[kChHalf];
+    const int h = threadIdx.x / kChHalf, j = threadIdx.x % kChHalf;      // h = 0: real parts, 1: imaginary
     const long long p = blockIdx.x;
     const bool st = j < kVpNS;
-    double scale = 0.0;
-    for (int s = 0; s < d.nsh; ++s) {
+    auto fetch_K = [&](int s) {                                         // of the step from shell s - 1 to s
+        const double* Ks = d.K + (long long)(s - 1) * kVpNS * kVpNS;
+        for (int e = 2 * threadIdx.x; e < kVpNS * kVpNS; e += 2 * kChSmallThreads) cp_async<16>(&sK[s & 1][e], Ks + e, true);
+        cp_async_commit();
+    };
+    auto max_of = [&](double v) {                                       // over the h = 0 threads
+        if (h == 0) red[j] = v;
         __syncthreads();
-        if (s > 0) {
-            const double* Ks = d.K + (long long)(s - 1) * kVpNS * kVpNS;
-            for (int e = j; e < kVpNS * kVpNS; e += kChSmallThreads) sK[e] = Ks[e];
+        for (int o = kChHalf / 2; o > 0; o >>= 1) {
+            if (h == 0 && j < o) red[j] = fmax(red[j], red[j + o]);
+            __syncthreads();
         }
-        double2 al = alin[(long long)s * NP + p];
-        for (int pc = 1; pc < npieces; ++pc) {
-            const double2 a2 = alin[((long long)pc * d.nsh + s) * NP + p];
-            al.x += a2.x; al.y += a2.y;
-        }
-        if (st) {
-            double2 zz = zp[((long long)s * kVpNS + j) * NP + p];
-            for (int pc = 1; pc < npieces; ++pc) {
-                const double2 z2 = zp[(((long long)pc * d.nsh + s) * kVpNS + j) * NP + p];
-                zz.x += z2.x; zz.y += z2.y;
-            }
-            const double uj = d.u[j];
-            zr_s[j] = fma(uj, al.x, zz.x);
-            zi_s[j] = fma(uj, al.y, zz.y);
+        const double m = red[0];
+        __syncthreads();
+        return m;
+    };
+    auto part = [&](const double2& v) { return h == 0 ? v.x : v.y; };
+    if (h == 0 && st) sw[j] = d.w[j];
+    const double uj = st ? d.u[j] : 0.0;
+    double scale = 0.0;
+    double zn = st ? part(zp[(long long)j * NP + p]) : 0.0, an = part(alin[p]);
+    for (int s = 0; s < d.nsh; ++s) {
+        if (st) z_s[h][j] = fma(uj, an, zn);
+        if (s + 1 < d.nsh) {                                            // the next shell's inputs on their way
+            fetch_K(s + 1);
+            zn = st ? part(zp[((long long)(s + 1) * kVpNS + j) * NP + p]) : 0.0;
+            an = part(alin[(long long)(s + 1) * NP + p]);
         }
         __syncthreads();
         if (j == 0) {
-            double mr = 0.0, mi = 0.0;
-            for (int i = 0; i < kVpNS; ++i) { mr = fma(d.w[i], zr_s[i], mr); mi = fma(d.w[i], zi_s[i], mi); }
-            s_mr = mr; s_mi = mi;
+            double m = 0.0;
+            for (int i = 0; i < kVpNS; ++i) m = fma(sw[i], z_s[h][i], m);
+            mn[h] = m;
         }
-        __syncthreads();
-        double zr = 0.0, zi = 0.0;
-        if (st) { zr = zr_s[j] - s_mr; zi = zi_s[j] - s_mi; }
-        red[j] = st ? zr : -1e300;
-        __syncthreads();
-        for (int o = kChSmallThreads / 2; o > 0; o >>= 1) {
-            if (j < o) red[j] = fmax(red[j], red[j + o]);
-            __syncthreads();
-        }
-        const double mx = red[0];
-        __syncthreads();
-        double nr = 0.0, ni = 0.0;
+        double g = 0.0;
         if (st) {
-            double gr, gi;
-            if (s == 0) { gr = d.w[j]; gi = 0.0; }
-            else {
-                gr = 0.0; gi = 0.0;
-                for (int i = 0; i < kVpNS; ++i) {
-                    const double kij = sK[i * kVpNS + j];
-                    gr = fma(kij, ar[i], gr); gi = fma(kij, ai[i], gi);
-                }
-            }
-            const double m = exp(zr - mx);
-            double sn, cs;
-            sincos(zi, &sn, &cs);
-            const double er = m * cs, ei = m * sn;
-            nr = gr * er - gi * ei;
-            ni = gr * ei + gi * er;
+            if (s == 0) g = h == 0 ? sw[j] : 0.0;
+            else
+                for (int i = 0; i < kVpNS; ++i) g = fma(sK[s & 1][i * kVpNS + j], al_s[h][i], g);
+            g_s[h][j] = g;
         }
-        red[j] = st ? nr * nr + ni * ni : 0.0;
         __syncthreads();
-        for (int o = kChSmallThreads / 2; o > 0; o >>= 1) {
-            if (j < o) red[j] = fmax(red[j], red[j + o]);
-            __syncthreads();
+        const double z = st ? z_s[h][j] - mn[h] : 0.0;
+        const double mx = max_of(st ? z : -1e300);
+        if (st) {
+            if (h == 0) ex_s[j] = exp(z - mx);
+            else sincos(z, &tr_s[j].y, &tr_s[j].x);
         }
-        const double nrm = sqrt(red[0]);
+        __syncthreads();
+        if (st) {
+            const double er = ex_s[j] * tr_s[j].x, ei = ex_s[j] * tr_s[j].y, gr = g_s[0][j], gi = g_s[1][j];
+            n_s[h][j] = h == 0 ? gr * er - gi * ei : gr * ei + gi * er;
+        }
+        __syncthreads();
+        const double nrm = sqrt(max_of(h == 0 && st ? n_s[0][j] * n_s[0][j] + n_s[1][j] * n_s[1][j] : 0.0));
         const double inv = 1.0 / nrm;
-        if (st) { ar[j] = nr * inv; ai[j] = ni * inv; }
-        scale += mx + log(nrm);
+        if (st) al_s[h][j] = n_s[h][j] * inv;
+        if (threadIdx.x < 32) scale += mx + log(nrm);
+        cp_async_wait<0>();
+        __syncthreads();
+    }
+    if (j == 0) {
+        double a = 0.0;
+        for (int i = 0; i < kVpNS; ++i) a += al_s[h][i];
+        mn[h] = a;
     }
     __syncthreads();
-    if (j == 0) {
-        double sr = 0.0, si = 0.0;
-        for (int i = 0; i < kVpNS; ++i) { sr += ar[i]; si += ai[i]; }
+    if (threadIdx.x == 0) {
+        const double sr = mn[0], si = mn[1];
         const long long o = (long long)kb * nq + p;
         out_re[o] = scale + 0.5 * log(sr * sr + si * si);
         out_im[o] = atan2(si, sr);
@@ -1073,7 +1086,12 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
             SGL_COUNT(1);
         }
         if (NP <= 4LL * kNumSMs) {
-            k_vp_chain_small<<<(unsigned)NP, kChSmallThreads, 0, st>>>(d, zp, al, NP, nq, kb, out_re, out_im, npieces);
+            const long long na = (long long)d.nsh * NP, nz = na * kVpNS;
+            if (npieces > 1) {
+                k_vp_sum_pieces<<<ceil_div(nz + na, 128), 128, 0, st>>>(zp, nz, al, na, npieces);
+                SGL_COUNT(1);
+            }
+            k_vp_chain_small<<<(unsigned)NP, kChSmallThreads, 0, st>>>(d, zp, al, NP, nq, kb, out_re, out_im);
             SGL_COUNT(1);
         } else if (Kff) {
             k_vp_chain_ff<<<ceil_div(NP, kCfPts), kCfThreads, sizeof(ChainShared), st>>>(d, Kff, zp, al, NP, nq, kb, out_re,
