@@ -249,6 +249,96 @@ k_vp_z(VpDevice d, const typename V2<TT>::T* __restrict__ e, const typename V2<T
         if (live[P]) alin[(long long)s * NP + pidx[P]] = make_double2(ALr[P], ALi[P]);
 }
 
+// ---- phase 1 of the mixed path on a line of points (the k-reach probes)
+// A warp takes a piece of a shell's cells for 32 points, a point per lane: cell indices and weights read 32 at a time and
+// broadcast, the table entries of eight cells in flight; sums as in k_vp_z (FP32 over 32 cells of a run, float-float over
+// the run, FP64 over the bounds).  Bound by the latency of the gathers from L2.  k_vp_z's 16 x 32 tiles hold a column or
+// a row of such points: 20 points, 0.77 M cells 0.84 and 0.75 -> 0.13 ms.
+constexpr int kZlThreads = 128;
+
+__global__ void __launch_bounds__(kZlThreads)
+k_vp_z_line(VpDevice d, const float2* __restrict__ e, const float2* __restrict__ Jt, int nk, int nq, double2* __restrict__ zp,
+            double2* __restrict__ alin, long long NP, int npieces) {
+    const int lane = threadIdx.x & 31, g = blockIdx.y * (kZlThreads / 32) + (threadIdx.x >> 5);
+    if (g >= d.nsh * npieces) return;
+    const int s = g / npieces, piece = g % npieces;
+    zp += (long long)piece * d.nsh * kVpNS * NP;
+    alin += (long long)piece * d.nsh * NP;
+    const long long p = (long long)blockIdx.x * 32 + lane;
+    const bool live = p < NP;
+    const int pp = live ? (int)p : 0;
+    const float2* ek = e + pp / nq;
+    const float2* jq = Jt + pp % nq;
+    double SAr = 0.0, SAi = 0.0, SBr = 0.0, SBi = 0.0, ALr = 0.0, ALi = 0.0;
+    int jcur = 0;
+    auto emit_to = [&](int jend) {
+        for (; jcur < jend; ++jcur) {
+            const double uj = d.u[jcur];
+            if (live) zp[((long long)s * kVpNS + jcur) * NP + p] = make_double2(fma(uj, SAr, SBr), fma(uj, SAi, SBi));
+        }
+    };
+    // an equal part of the shell's cells (a run may span pieces: its contribution is additive), cut at 32 cells
+    const int rs0 = d.sh_run[s], rs1 = d.sh_run[s + 1];
+    const long long sc0 = d.run_cell[rs0], sn = d.run_cell[rs1] - sc0;
+    const long long cb = sc0 + sn * piece / npieces, ce = sc0 + sn * (piece + 1) / npieces;
+    int r0 = rs0, hi_r = rs1;                                // the run that holds cb
+    while (hi_r - r0 > 1) {
+        const int mid = (r0 + hi_r) >> 1;
+        if (d.run_cell[mid] <= cb) r0 = mid; else hi_r = mid;
+    }
+    for (int r = r0; r < rs1; ++r) {
+        const long long rc = d.run_cell[r], c0 = max(cb, rc), c1 = min(ce, d.run_cell[r + 1]);
+        if (rc >= ce) break;
+        if (c0 >= c1) continue;
+        float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+        for (long long base = c0; base < c1; base += 32) {
+            const int cnt = (int)min(32LL, c1 - base);
+            const int cu = lane < cnt ? d.cu[base + lane] : 0;
+            const float2 w = lane < cnt ? d.wabf[base + lane] : make_float2(0.f, 0.f);
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int b = 0; b < cnt; b += 8) {
+                float2 ev[8], jv[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const long long c = __shfl_sync(0xffffffffu, cu, b + i);      // (0 beyond the run's cells)
+                    ev[i] = __ldg(ek + c * nk);
+                    jv[i] = __ldg(jq + c * nq);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (b + i >= cnt) break;
+                    const float wa = __shfl_sync(0xffffffffu, w.x, b + i), wb = __shfl_sync(0xffffffffu, w.y, b + i);
+                    const float Fr = ev[i].x * jv[i].x + jv[i].y;                 // (cos - 1) J + (J - 1)
+                    const float Fi = ev[i].y * jv[i].x;                           // sin J
+                    v[0] += wa * Fr; v[1] += wa * Fi;
+                    v[2] += wb * Fr; v[3] += wb * Fi;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ff_acc(hi[i], lo[i], v[i]);
+        }
+        const double Ar = (double)hi[0] + (double)lo[0], Ai = (double)hi[1] + (double)lo[1];
+        const double Br = (double)hi[2] + (double)lo[2], Bi = (double)hi[3] + (double)lo[3];
+        const int kind = d.run_kind[r], bound = d.run_bound[r];
+        if (kind == 0) {                                   // linear: u_j A (intercept dropped)
+            ALr += Ar; ALi += Ai;
+        } else if (kind == 1) {                            // left: states >= lo, anchored at u_lo
+            emit_to(bound);
+            const double ub = d.u[bound];
+            SAr += Ar; SAi += Ai;
+            SBr += fma(-ub, Ar, Br); SBi += fma(-ub, Ai, Bi);
+        } else {                                           // right: states <= hi, anchored at u_hi (as in k_vp_z)
+            emit_to(bound + 1);
+            const double ub = d.u[bound];
+            ALr += Ar; ALi += Ai;
+            SAr -= Ar; SAi -= Ai;
+            SBr += fma(ub, Ar, -Br); SBi += fma(ub, Ai, -Bi);
+        }
+    }
+    emit_to(kVpNS);
+    if (live) alin[(long long)s * NP + p] = make_double2(ALr, ALi);
+}
+
 // ---- phase 1 of the mixed path on a grid of points
 // F splits into e_c(k) J_c(q), of both axes, and J_c(q) - 1, of k_gamma alone: the second part of every run is summed
 // once per q (k_vp_jm), and per (cell, point) only two packed FMAs remain, J times (w a e_re, w a e_im) and
@@ -998,7 +1088,7 @@ k_vp_chain_small(VpDevice d, const double2* __restrict__ zp, const double2* __re
     }
 }
 
-// the mixed path's grid kernel pays from a few tiles of points on; the k-reach probe lines keep k_vp_z
+// the mixed path's grid kernel pays from a few tiles of points on
 bool vp_mixed_grid(int precision, int nk, int nq) { return precision != SGL_FP64 && nk >= 8 && nq >= 32; }
 static int vp_nqp(int nq) { return ceil_div(nq, kMzQ) * kMzQ; }
 
@@ -1019,7 +1109,15 @@ int vp_rows_per_pass(int nsh, int nk, int nq, size_t z_cap_bytes) {
     return (int)((nk + passes - 1) / passes);
 }
 
+// lines of points of the mixed path (the grid kernel's tiles and k_vp_z's would be mostly empty)
+static bool vp_line(int precision, int nk, int nq) { return precision != SGL_FP64 && (nk == 1 || nq == 1) && (long long)nk * nq <= 4LL * kNumSMs; }
+
 int vp_pieces(int precision, int nsh, int rows, int nq) {
+    if (vp_line(precision, rows, nq)) {
+        // sixteen warps per SM
+        const long long base = (long long)ceil_div((long long)rows * nq, 32) * nsh;
+        return (int)std::max(1LL, std::min(128LL, 16LL * kNumSMs / base));
+    }
     if (vp_mixed_grid(precision, rows, nq)) {
         // two CTAs per SM: at least four waves, so that the last one costs at most a fifth
         const long long base = (long long)(vp_nqp(nq) / kMzQ) * ceil_div(rows, kMzK) * nsh;
@@ -1079,6 +1177,10 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
         } else if (grid) {
             k_vp_z_mixed<<<dim3(nqp / kMzQ, ceil_div(nkc, kMzK), d.nsh * npieces), kMzThreads, 0, st>>>(
                 d, (const float2*)e, J, jm, nk, nq, nqp, kb, nkc, zp, al, NP, npieces);
+            SGL_COUNT(1);
+        } else if (vp_line(precision, nk, nq)) {
+            const dim3 gl(ceil_div(NP, 32), ceil_div((long long)d.nsh * npieces, kZlThreads / 32));
+            k_vp_z_line<<<gl, kZlThreads, 0, st>>>(d, (const float2*)e, (const float2*)Jt, nk, nq, zp, al, NP, npieces);
             SGL_COUNT(1);
         } else {
             k_vp_z<float><<<g1, kZThreads, 0, st>>>(d, (const float2*)e, (const float2*)Jt, nk, nq, kb, nkc, zp, al, NP,

@@ -54,3 +54,28 @@ def test_large_phases_take_the_fp64_sine():
     k, q = np.linspace(0.0, 3.0, 16), np.linspace(0.0, 2.0, 40)
     a, b = e.vp_lnR(k, q, SGL_FP64), e.vp_lnR(k, q, SGL_MIXED)
     assert np.all(np.abs(np.exp(a - b) - 1) <= 1e-5 + 2e-8 * np.abs(a))
+
+
+@pytest.mark.parametrize("n", [1, 2, 20, 31, 32, 33, 608, 609])
+@pytest.mark.parametrize("shells", [1, 6])
+@pytest.mark.parametrize("axis", ["k", "q"])
+def test_lines_of_points(n, shells, axis):
+    """The probes' lines: part of a warp, whole warps, the last count that takes the line kernel and the next."""
+    x = np.geomspace(1.0, 900.0, n)
+    d = _closure(shells)
+    if axis == "k":
+        _compare(d, x, np.zeros(1))
+        _compare(d, x, np.full(1, 300.0))
+    else:
+        _compare(d, np.zeros(1), x)
+
+
+def test_lines_of_right_and_linear_runs():
+    d = _closure(3)
+    ns = d["u"].size
+    clipped = d["gc"] != 0
+    m = dict(d, K=d["K"][:, ::-1, ::-1].copy(), w=d["w"][::-1].copy(), ga=-d["ga"],
+             glo=np.where(clipped, ns - 1 - d["ghi"], d["glo"]).astype(np.int32),
+             ghi=np.where(clipped, ns - 1 - d["glo"], d["ghi"]).astype(np.int32))
+    _compare(m, np.linspace(0.0, 900.0, 20), np.full(1, 40.0))
+    _compare(m, np.full(1, 90.0), np.linspace(0.0, 700.0, 50))
