@@ -541,13 +541,13 @@ inline sgl_status check_dev_err(sgl_ctx* ctx) {
 // drain = true: the drained-accumulation kernel (TMEM sums folded into TwoSum running sums every
 // 64 products), tiles of at most tc_drain_bn() columns
 inline sgl_status run_tc_gemms(sgl_ctx* ctx, std::vector<TcGemmDesc>& d, const std::string& tag, int parts,
-                               bool drain = false) {
+                               bool drain = false, int bn_max = 256) {       // 256: the TMEM columns of one tile
     if (d.empty()) return SGL_OK;
     std::vector<TcPackDesc> pk(2 * d.size());
     int tiles = 0;
     long long quads = 0;
     const long long pfl = tc_gemm_plan(d.data(), (int)d.size(), parts, pk.data(), &tiles, &quads, true,
-                                       drain ? tc_drain_bn() : 256);     // 256: the TMEM columns of one tile
+                                       drain ? tc_drain_bn() : bn_max);
     DBUF(dd, TcGemmDesc, "tc_desc_" + tag, d.size());
     DBUF(dp, TcPackDesc, "tc_pack_" + tag, pk.size());
     DBUF(packed, float, "tc_packed", std::max<long long>(pfl, 1));

@@ -1,8 +1,8 @@
-"""sgl_mlp_layer, the K-sliced sgl_gemm_bf16 and the column sums at the edges of their tiles, against the same
+"""sgl_mlp_layer, sgl_gemm_bf16 with a long K and the column sums at the edges of their tiles, against the same
 arithmetic in torch FP64 on the same BF16-rounded operands.
 
 Bounds: products of BF16 values are exact in FP32 and accumulate over K terms in FP32 (2^-23 each, truncation
-included): 2^-23 sqrt(K) of the sum of magnitudes is typical, K 2^-23 the worst; 32 x 2^-23 = 4e-6 of it is asserted (slices of 4096 terms stay below it on these inputs' random signs).
+included): 2^-23 sqrt(K) of the sum of magnitudes is typical, K 2^-23 the worst; 32 x 2^-23 = 4e-6 of it is asserted (sums stay below it on these inputs' random signs).
 Column sums are FP64 sums rounded to FP32."""
 import numpy as np
 import pytest
@@ -57,7 +57,7 @@ def test_layer_gradient(M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(256, 256, 8191), (256, 256, 8192), (8, 256, 16384), (256, 2, 12301), (130, 300, 9000)])
-def test_sliced_weight_gradient(M, N, K):
+def test_weight_gradient(M, N, K):
     torch, e, r = _setup(K)
     A, B = r(K, M), r(K, N)
     C = torch.zeros((M, N), device="cuda")
