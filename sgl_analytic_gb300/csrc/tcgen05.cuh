@@ -116,6 +116,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity
     return true;
 }
 
+// One answer for a converged warp.  A bounded wait can run out for some of a warp's lanes only (each reads the clock and
+// the failure flag for itself); where shuffles, votes or tcgen05.ld follow, the lanes must stop or go on together.
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
+
 // two 16-column loads (e.g. the same lanes of two accumulators) under one wait
 __device__ __forceinline__ void tmem_ld16x2(uint32_t ta, uint32_t tb, float* va, float* vb) {
     uint32_t r[32];

@@ -282,8 +282,8 @@ k_xi_fused(XiFusedArgs a) {
                 }
             }
             const int kb = b / kXfBlocks, pb = b % kXfBlocks, s = kb % kXfStages;
-            // its stage must have been consumed by the MMAs of kb - S
-            if (*s_fail || (kb >= kXfStages && !wait_consumed(kb - kXfStages))) {
+            // its stage must have been consumed by the MMAs of kb - S (the warp stops or goes on as one)
+            if (!warp_all(!*s_fail && (kb < kXfStages || wait_consumed(kb - kXfStages)))) {
                 *s_fail = 1;
                 break;
             }
