@@ -281,7 +281,8 @@ k_oz_gemm(const OzGemmDesc* __restrict__ descs, int nprob, const unsigned char* 
         const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * kCols);
         bool ok = true;
         for (int blk = 0; blk < nblk && ok; ++blk) {
-            if (*s_fail || !mbar_wait_bounded(accf, (uint32_t)(blk & 1))) { ok = false; break; }
+            ok = warp_all(!*s_fail && mbar_wait_bounded(accf, (uint32_t)(blk & 1)));
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int c0 = 0; c0 < kCols; c0 += 16) {
