@@ -430,7 +430,8 @@ k_tc_gemm_drain(const TcGemmDesc* __restrict__ descs, int nprob, const float* __
         bool ok = true;
         for (int blk = 0; blk < nblk && ok; ++blk) {
             const int a = blk & 1;
-            if (*s_fail || !mbar_wait_bounded(accf(a), (uint32_t)((blk >> 1) & 1))) { ok = false; break; }
+            ok = warp_all(!*s_fail && mbar_wait_bounded(accf(a), (uint32_t)((blk >> 1) & 1)));
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int c0 = 0; c0 < kTcDrainBN; c0 += 16) {

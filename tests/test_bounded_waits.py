@@ -63,6 +63,6 @@ def _unvoted(path):
     return bad
 
 
-@pytest.mark.parametrize("name", ["xi_fused.cu", "mlp_fused.cu", "oz_gemm.cu"])
+@pytest.mark.parametrize("name", ["xi_fused.cu", "mlp_fused.cu", "oz_gemm.cu", "tc_gemm.cu"])
 def test_lanes_of_a_warp_agree_on_a_wait_that_ran_out(name):
     assert _unvoted(CSRC / name) == []
