@@ -160,6 +160,7 @@ k_tc_gemm(const TcGemmDesc* __restrict__ descs, int nprob, const float* __restri
     const long long a_part = (long long)d.Mpad * kTcBK, b_part = (long long)d.Npad * kTcBK;
     const uint32_t a_bytes = kTcAbytes, b_bytes = (uint32_t)bn * kTcBK * 4;
 
+    int issued = 0;                            // K blocks whose copies the producer issued
     if (tid == 0 && nkb > 0) {
         // producer: one bulk copy per operand part and K block
         for (int kb = 0; kb < nkb; ++kb) {
@@ -169,6 +170,7 @@ k_tc_gemm(const TcGemmDesc* __restrict__ descs, int nprob, const float* __restri
                 break;
             }
             const uint32_t st = sbase + s * Cfg::kStageBytes;
+            issued = kb + 1;
             mbar_expect_tx(bar + 8 * s, NP * (a_bytes + b_bytes));
             const float* a = Ap + ((long long)NP * kb) * a_part + (long long)(i0 >> 3) * 128;
             const float* b = Bp + ((long long)NP * kb) * b_part + (long long)(j0 >> 3) * 128;
@@ -278,6 +280,8 @@ k_tc_gemm(const TcGemmDesc* __restrict__ descs, int nprob, const float* __restri
         }
     } else if (tid == 0) {
         atomicExch(err, 1);
+        // no bulk copy may outlive the CTA: waits (bounded) for those of the last stages
+        for (int kb = issued > S ? issued - S : 0; kb < issued; ++kb) mbar_wait_bounded(bar + 8 * (kb % S), (uint32_t)((kb / S) & 1));
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -29,7 +29,7 @@
 // hidden), last products 5k, squares 5k.  One launch: 1.55 -> 1.36 ms (three warps per 4-p block with a group barrier and
 // a bulk copy per chunk of entries, squares with a test per column: 147k cycles a CTA).
 // The summation order of T over entries and of the squares over rr is that of the unfused kernels.
-// Every wait is bounded; a wait that runs out sets *err and the CTA skips to its TMEM release.
+// Every wait is bounded; a wait that runs out sets *err, and the CTA waits for its copies in flight and releases its TMEM.
 #include "kernels.cuh"
 #include "tcgen05.cuh"
 
@@ -227,6 +227,7 @@ k_xi_fused(XiFusedArgs a) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *(volatile uint32_t*)(xsm + boff + 8 * kNBar);
 
+    int issued = 0;                                      // K blocks whose E copy was issued
     if (warp < kXfProdWarps && nkb > 0) {
         // ---- T producers.  Lane (u, rg, jh): p = 4 b + u of block b, row quads rg, rg + 4, rg + 8, columns 4 jh .. + 3;
         // an entry's sums run over the entries in order
@@ -325,6 +326,7 @@ k_xi_fused(XiFusedArgs a) {
                 *s_fail = 1;
                 break;
             }
+            issued = kb + 1;
             mbar_expect_tx(full(s), kXfABytes);
             bulk_g2s(sbase + s * kXfStageBytes, Eg + (long long)kb * (kXfABytes / 4), kXfABytes, full(s));
         }
@@ -396,8 +398,11 @@ k_xi_fused(XiFusedArgs a) {
                 if (n < nk && j < nkg) a.part[((long long)g * nkg + j) * nk + n] = s;
             }
         }
-    } else if (tid == 0) {
-        atomicExch(a.err, 1);
+    } else {
+        if (tid == 0) atomicExch(a.err, 1);
+        // no bulk copy may outlive the CTA: waits for those of the last stages, bounded (a barrier whose producers gave up
+        // never completes, but by then its copy has long landed)
+        for (int kb = max(0, issued - kXfStages); kb < issued; ++kb) mbar_wait_sleep(full(kb % kXfStages), (uint32_t)((kb / kXfStages) & 1));
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

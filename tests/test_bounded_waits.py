@@ -66,3 +66,14 @@ def _unvoted(path):
 @pytest.mark.parametrize("name", ["xi_fused.cu", "mlp_fused.cu", "oz_gemm.cu", "tc_gemm.cu"])
 def test_lanes_of_a_warp_agree_on_a_wait_that_ran_out(name):
     assert _unvoted(CSRC / name) == []
+
+
+def test_a_cta_that_gave_up_waits_for_its_bulk_copies():
+    """A bulk copy that lands after its CTA has ended writes into the next one's shared memory.  Every kernel that issues
+    them has a loop of waits over those issued but not taken, after the roles (mlp_fused: at the end of the copy role)."""
+    wait = re.compile(r"for \([^{;]*;[^{;]*(?:\bissued\b|\bj >= 0\b)[^{;]*;[^{;]*\)\s*(?:if \(!)?mbar_wait_(?:bounded|sleep)\(")
+    for name in ("xi_fused.cu", "mlp_fused.cu", "oz_gemm.cu", "tc_gemm.cu"):
+        s = _code(CSRC / name)
+        for kernel in re.split(r"__global__", s)[1:]:
+            if "bulk_g2s(" in kernel:
+                assert wait.search(kernel, kernel.rindex("bulk_g2s(")), (name, " ".join(kernel[:120].split()))
