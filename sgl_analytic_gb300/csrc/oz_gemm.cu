@@ -57,13 +57,15 @@ __device__ __forceinline__ int find_desc(const D* d, int n, long long v, F begin
 }
 
 // Scales: the largest biased exponent of a row, each element's first shifted by the k scales' sign * (kexp - 1023), kept as
-// kOzBias + exponent (0: a row of zeros); kOzNan: the row holds an infinity or a NaN
-constexpr int kOzBias = 8192, kOzNan = 1 << 20;
+// kOzBias + exponent (0: a row of zeros); kOzNan: the row holds an infinity or a NaN.  A k scale is that of the finite
+// elements of A's column; where it has none but zeros, row k of B adds nothing to any finite output, so it is cut to zero
+// digits and does not enter the scales of B's columns (unscaled, it would push the rows that count out of their digits).
+constexpr int kOzBias = 8192, kOzNan = 1 << 20, kOzDead = 1 << 24;
 
 __device__ __forceinline__ int oz_shift(const OzPackDesc& d, const int* scale, int k) {
     if (d.k_sign == 0) return 0;
     const int s = scale[d.k_off + k];
-    return s == 0 || s >= kOzNan ? 0 : d.k_sign * (s - kOzBias - 1023);
+    return s == 0 ? kOzDead : d.k_sign * (s - kOzBias - 1023);
 }
 
 __global__ void __launch_bounds__(256) k_oz_scale(const OzPackDesc* __restrict__ descs, int n, int* __restrict__ scale) {
@@ -75,7 +77,8 @@ __global__ void __launch_bounds__(256) k_oz_scale(const OzPackDesc* __restrict__
     const int k1 = min(d.K, k0 + kOzScaleK);
     auto exponent = [&](double v, int shift) {
         const int e = (__double2hiint(v) >> 20) & 0x7ff;
-        return v == 0.0 ? 0 : (e == 0x7ff ? kOzNan : kOzBias + max(e, 1) + shift);
+        if (e == 0x7ff) return d.k_sign == 0 ? 0 : kOzNan;
+        return v == 0.0 || shift == kOzDead ? 0 : kOzBias + max(e, 1) + shift;
     };
     __shared__ int s_shift[kOzScaleK];
     for (int k = threadIdx.x; k < k1 - k0; k += 256) s_shift[k] = oz_shift(d, scale, k0 + k);
@@ -122,8 +125,9 @@ __global__ void __launch_bounds__(256) k_oz_pack(const OzPackDesc* __restrict__ 
         long long m = bits & 0xfffffffffffffLL;
         if (ex > 0) m |= 1LL << 52;
         // to 55 bits for the row's largest exponent
-        const int sh = max(ex, 1) + (k < d.K ? oz_shift(d, scale, k) : 0) + kOzBias - emax + 2;
-        if (m == 0 || emax >= kOzNan) m = 0;
+        const int shift = k < d.K ? oz_shift(d, scale, k) : 0;
+        const int sh = max(ex, 1) + shift + kOzBias - emax + 2;
+        if (m == 0 || emax >= kOzNan || shift == kOzDead) m = 0;
         else if (sh >= 0) m <<= sh;                             // 0 .. 2
         else m = sh < -56 ? 0 : (m + (1LL << (-sh - 1))) >> -sh;
         if (bits < 0) m = -m;
