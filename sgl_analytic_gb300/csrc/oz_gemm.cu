@@ -57,7 +57,8 @@ __device__ __forceinline__ int find_desc(const D* d, int n, long long v, F begin
 }
 
 // Scales: the largest biased exponent of a row, each element's first shifted by the k scales' sign * (kexp - 1023), kept as
-// kOzBias + exponent (0: a row of zeros); kOzNan: the row holds an infinity or a NaN.  A k scale is that of the finite
+// kOzBias + exponent (0: a row of zeros); kOzNan: the row holds an infinity or a NaN (its outputs are summed by plain
+// FMAs in the epilogue, so that infinities and NaN come out as of an FP64 product).  A k scale is that of the finite
 // elements of A's column; where it has none but zeros, row k of B adds nothing to any finite output, so it is cut to zero
 // digits and does not enter the scales of B's columns (unscaled, it would push the rows that count out of their digits).
 constexpr int kOzBias = 8192, kOzNan = 1 << 20, kOzDead = 1 << 24;
@@ -175,6 +176,12 @@ __device__ __forceinline__ double oz_value(long long hi, long long lo, int e, bo
     s = normal ? s : 0;
     const long long v = (((long long)(E + s - 1) << 52) + (long long)m) | (neg ? (long long)(1ULL << 63) : 0);
     return __longlong_as_double(H == 0 ? 0 : v);
+}
+
+__device__ __noinline__ double oz_plain_sum(const double* a, long long a_cs, const double* b, long long b_rs, int K) {
+    double acc = 0.0;
+    for (int k = 0; k < K; ++k) acc = fma(a[(long long)k * a_cs], b[(long long)k * b_rs], acc);
+    return acc;
 }
 
 __global__ void __launch_bounds__(kOzThreads, 1)
@@ -326,7 +333,10 @@ k_oz_gemm(const OzGemmDesc* __restrict__ descs, int nprob, const unsigned char* 
                     const int eb = __shfl_sync(0xffffffffu, ebs, c);
                     double* o = s_out + lane * (kCols + 1) + c;
                     if (odd >> c & 1) *o = scalbn(*o, ea + eb - 2 * kOzBias - 2106);
-                    if (ea >= kOzNan || eb >= kOzNan) *o = __longlong_as_double(0x7ff8000000000000LL);
+                    // an infinity or a NaN in the row or the column: the sum of products as FP64 FMAs form it
+                    const int jc = j - lane + c;
+                    if ((ea >= kOzNan || eb >= kOzNan) && r0 + lane < d.M && jc < d.N)
+                        *o = oz_plain_sum(d.A + (long long)(r0 + lane) * d.a_rs, d.a_cs, d.B + (long long)jc * d.b_cs, d.b_rs, d.K);
                 }
             __syncwarp();
             const int nr = j < d.N ? min(32, d.M - r0) : 0;

@@ -3,6 +3,8 @@ left operand, with k_gamma as the product's inner index."""
 import numpy as np
 import pytest
 
+from tests.conftest import GOLDEN
+
 pytestmark = pytest.mark.gpu
 
 GRID = dict(nk_k=331, nk_g=1203, n_kap=601, n_gam=257, k_k_max=120.0, k_g_max=110.0, kap_min=-0.3, kap_max=0.99,
@@ -34,3 +36,26 @@ def test_empty_columns_beside_small_ones(scale, empty):
     P, m = Engine(0).invert_phi(phi * scale, GRID, X, precision=SGL_FP64)
     ref = _oracle(kk, kg, phi)
     assert np.max(np.abs(P * (m["norm"] / scale) - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_an_infinity_stays_one():
+    """An infinite row element of the xi groups: infinities and NaN where FP64 products have them, as the same rows of a
+    grid too small for the slices (below 0.4 GFLOP) show."""
+    from sgl_analytic_gb300 import Lam, Population
+    from sgl_analytic_gb300._lib import SGL_FP64
+    pop = Population.load(GOLDEN / "pop_zs1_sub.npz")
+    rng = np.random.default_rng(5)
+    n_k, n_g = pop.ce_k.size - 1, pop.ce_g.size - 1
+    idx = np.concatenate([ik * n_g + np.sort(rng.choice(n_g, 12, replace=False)) for ik in range(200)]).astype(np.int32)
+    rows = rng.standard_normal((36, idx.size + 1)) * 1e-2
+    rows[7, 40] = np.inf
+    pop.xg_m, pop.xg_nrow, pop.xg_nidx = np.array([1], np.int32), np.array([36], np.int32), np.array([idx.size], np.int32)
+    pop.xg_idx, pop.xg_rows = idx, rows.ravel()
+    lam = Lam(pop, xi=True, xi_prune=0.0)
+    kk, kg = np.linspace(0.0, 900.0, 101), np.linspace(0.0, 700.0, 101)          # 0.58 GFLOP
+    sel = np.array([0, 1, 50, 100])
+    q, few = lam.engine.xi_term(kk, kg, SGL_FP64), lam.engine.xi_term(kk[sel], kg, SGL_FP64)
+    assert np.isinf(few.imag).any()
+    for a, b in ((q.real[sel], few.real), (q.imag[sel], few.imag)):
+        assert np.array_equal(np.isnan(a), np.isnan(b))
+        assert np.array_equal(a[np.isinf(a)], b[np.isinf(b)])
