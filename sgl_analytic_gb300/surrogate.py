@@ -120,11 +120,12 @@ class MLP:
                                     crs, ccs, 1.0), "sgl_gemm_bf16")
 
     def forward(self, X, keep=False):
-        """X: (n, 8) float32 device tensor -> (n, 2); keep=True stores activations for backward."""
+        """X: (n, 8) device tensor, float32 (other types are converted) -> (n, 2); keep=True stores activations for
+        backward."""
         torch, e = self.torch, self.eng
         n = X.shape[0]
         with torch.cuda.stream(self.stream):
-            A = X.contiguous()
+            A = X.to(torch.float32).contiguous()                   # the kernels read packed FP32 rows
             acts, pre = [A], []
             for l, (W, b) in enumerate(zip(self.W, self.b)):
                 a, c = W.shape
