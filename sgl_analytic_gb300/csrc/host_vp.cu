@@ -32,11 +32,13 @@ sgl_status vp_lnR_device(sgl_ctx* ctx, int precision, const double* d_kv, int nk
     Timed t(ctx, precision == SGL_FP64 ? "vp_lnR_f64" : "vp_lnR_mixed", pts * (double)D.ncells * 12.0,
             pts * D.nsh * 49 * 16.0 * 2);
     float2* Kff = nullptr;
+    unsigned char* redo = nullptr;
     if (precision == SGL_MIXED) {
         Kff = dbuf<float2>(ctx, "vp_Kff", std::max<size_t>(1, (size_t)(D.nsh - 1) * 48 * 48));
-        if (!Kff) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (vp)");
+        redo = dbuf<unsigned char>(ctx, "vp_redo", (size_t)rows * nq);
+        if (!Kff || !redo) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (vp)");
     }
-    launch_vp_lnR(precision, D, d_kv, nk, d_qv, nq, tables, (double2*)zb, rows, d_re, d_im, ctx->stream, pieces, Kff);
+    launch_vp_lnR(precision, D, d_kv, nk, d_qv, nq, tables, (double2*)zb, rows, d_re, d_im, ctx->stream, pieces, Kff, redo);
     CKLAUNCH();
     return SGL_OK;
 }

@@ -318,7 +318,8 @@ size_t vp_table_bytes(int precision, int U, int nk, int nq, int nruns);
 int vp_rows_per_pass(int nsh, int nk, int nq, size_t z_cap_bytes);
 void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, const double* qv, int nq, void* tables,
                    double2* zbuf, int rows_per_pass, double* out_re, double* out_im, cudaStream_t st, int npieces = 1,
-                   float2* Kff = nullptr);      // Kff (mixed; (nsh - 1) 48^2): scratch of the float-float chain
+                   float2* Kff = nullptr, unsigned char* redo = nullptr);
+                                                // Kff (mixed; (nsh - 1) 48^2), redo (a pass's points): the float-float chain's
 // pieces per shell for the phase-1 kernel so that a small point grid still fills the GPU
 int vp_pieces(int precision, int nsh, int rows, int nq);
 

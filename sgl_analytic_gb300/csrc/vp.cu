@@ -611,7 +611,7 @@ k_vp_z_mixed(VpDevice d, const float2* __restrict__ e, const float* __restrict__
 
 __global__ void __launch_bounds__(kChPts)
 k_vp_chain(VpDevice d, const double2* __restrict__ zp, const double2* __restrict__ alin, long long NP, int nq, int kb,
-           double* __restrict__ out_re, double* __restrict__ out_im, int npieces) {
+           double* __restrict__ out_re, double* __restrict__ out_im, int npieces, const unsigned char* __restrict__ only) {
     extern __shared__ __align__(16) unsigned char vsm[];
     double (*ar)[kChPts] = (double (*)[kChPts])vsm;                       // alpha (normalised)
     double (*ai)[kChPts] = (double (*)[kChPts])(vsm + 1 * kVpNS * kChPts * 8);
@@ -620,7 +620,11 @@ k_vp_chain(VpDevice d, const double2* __restrict__ zp, const double2* __restrict
     double* sK = (double*)(vsm + 4 * kVpNS * kChPts * 8);                    // K[s-1], 48 x 48
     const int t = threadIdx.x;
     const long long p = (long long)blockIdx.x * kChPts + t;
-    const bool live = p < NP;                  // dead threads only help stage K
+    bool live = p < NP;                        // dead threads only help stage K
+    if (only) {                                // not NULL: the points marked there
+        live = live && only[p] != 0;
+        if (!__syncthreads_or(live)) return;
+    }
     double scale = 0.0;
     for (int s = 0; s < d.nsh; ++s) {
         if (s > 0) {
@@ -705,6 +709,10 @@ k_vp_chain(VpDevice d, const double2* __restrict__ zp, const double2* __restrict
 // two, which is exact.  CTA: 32 points; phase A a thread per (point, 8 states): z, e^z into shared memory; phase B a thread
 // per (4 states, 2 points): alpha' = K^T alpha, times e^z.  409 x 109 points, 24 shells: 19.7 -> 3.7 ms; ln R differs from the FP64
 // path by the same 6e-12 (1 + |ln R|) as with the FP64 chain.
+// Range: every operation is exact to 2^-48 or to a few 2^-149 of the largest state, and a state that is small now can be the
+// largest later, when the others have been scaled down by 2^-E in all (E: the renormalisations' exponents, which only grow
+// where z spreads).  The transitions conserve the sum of such errors, so they reach at most 48 x 8 x shells x 2^(E - 149) of
+// the result: 5e-14 at E = 90 and 64 shells.  Points with more are marked, and k_vp_chain does them over in FP64.
 constexpr int kCfPts = 32, kCfThreads = 192;
 
 typedef unsigned long long P2;
@@ -739,10 +747,11 @@ __device__ __forceinline__ ff ff_reduce(ff x, float q, float c1, float c2h, floa
     return ff_quick(s.hi, s.lo + ((x.lo - e) - q * c2l));
 }
 
-// e^x, x <= 0: x = n ln 2 + r, 1 + r + r^2 / 2 + r^3 / 6 in float-float, the rest (6e-4 of the value) in FP32
+// e^x, x <= 0: x = n ln 2 + r, 1 + r + r^2 / 2 + r^3 / 6 in float-float, the rest (6e-4 of the value) in FP32; results down
+// to the subnormal numbers, 0 below 2^-150
 __device__ __forceinline__ ff ff_exp(ff x) {
     ff z = {0.f, 0.f};
-    if (x.hi < -86.f) return z;
+    if (x.hi < -104.f) return z;
     const float n = rintf(x.hi * 1.44269504088896341f);
     const ff r = ff_reduce(x, n, 0.693359375f, -2.12194442e-4f, 1.64659497e-12f);
     float t = fmaf(r.hi, 1.f / 3628800.f, 1.f / 362880.f);
@@ -759,9 +768,10 @@ __device__ __forceinline__ ff ff_exp(ff x) {
     v = ffx_add(h, v);
     v = ffx_add(r, v);
     v = ffx_add(one, v);
-    const float sc = __int_as_float(((int)n + 127) << 23);           // n >= -125
-    v.hi *= sc;
-    v.lo *= sc;
+    const int e1 = (int)n >> 1, e2 = (int)n - e1;                    // n >= -151: two normal factors
+    const float s1 = __int_as_float((e1 + 127) << 23), s2 = __int_as_float((e2 + 127) << 23);
+    v.hi = v.hi * s1 * s2;
+    v.lo = v.lo * s1 * s2;
     return v;
 }
 
@@ -802,18 +812,21 @@ struct ChainShared {
     double red[6][kCfPts][2];
     double mean[kCfPts][2], mx[kCfPts], scale[kCfPts];
     unsigned big[kCfPts];
+    int down[kCfPts];                          // E: exponents of the renormalisations, summed
 };
+constexpr int kCfMaxDown = 90;
 
 __global__ void __launch_bounds__(kCfThreads, 2)
 k_vp_chain_ff(VpDevice d, const float2* __restrict__ Kff, const double2* __restrict__ zp, const double2* __restrict__ alin,
-              long long NP, int nq, int kb, double* __restrict__ out_re, double* __restrict__ out_im, int npieces) {
+              long long NP, int nq, int kb, double* __restrict__ out_re, double* __restrict__ out_im, int npieces,
+              unsigned char* __restrict__ redo) {
     extern __shared__ __align__(16) unsigned char vsm[];
     ChainShared& S = *reinterpret_cast<ChainShared*>(vsm);
     const int t = threadIdx.x, pa = t % kCfPts, ja = t / kCfPts;             // phase A: point, states 8 ja .. 8 ja + 7
     const int pb = t % 16, jb = 4 * (t / 16);                                // phase B: points pb, pb + 16, states jb .. jb + 3
     const long long p0 = (long long)blockIdx.x * kCfPts, p = p0 + pa;
     const bool live = p < NP;
-    if (t < kCfPts) S.scale[t] = 0.0;
+    if (t < kCfPts) { S.scale[t] = 0.0; S.down[t] = 0; }
     const P2 m1 = f32x2_pack(-1.f, -1.f);
     for (int s = 0; s < d.nsh; ++s) {
         __syncthreads();                       // the previous shell's readers of alpha, K and the reductions are done
@@ -964,7 +977,11 @@ k_vp_chain_ff(VpDevice d, const float2* __restrict__ Kff, const double2* __restr
                 S.alpha[jb + q][pb + 16 * x] = make_float4(v.x * sc, v.y * sc, v.z * sc, v.w * sc);
             }
         }
-        if (t < kCfPts) S.scale[t] += S.mx[t] + max(-126, min(126, (int)(S.big[t] >> 23) - 126)) * 0.6931471805599453;
+        if (t < kCfPts) {
+            const int ex = max(-126, min(126, (int)(S.big[t] >> 23) - 126));
+            S.scale[t] += S.mx[t] + ex * 0.6931471805599453;
+            S.down[t] += max(0, -ex);
+        }
     }
     __syncthreads();
     if (t < kCfPts && live) {
@@ -974,6 +991,7 @@ k_vp_chain_ff(VpDevice d, const float2* __restrict__ Kff, const double2* __restr
             sr += (double)v.x + (double)v.z;
             si += (double)v.y + (double)v.w;
         }
+        redo[p] = S.down[t] > kCfMaxDown;
         const long long o = (long long)kb * nq + p;
         out_re[o] = S.scale[t] + 0.5 * log(sr * sr + si * si);
         out_im[o] = atan2(si, sr);
@@ -1129,7 +1147,8 @@ int vp_pieces(int precision, int nsh, int rows, int nq) {
 }
 
 void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, const double* qv, int nq, void* tables,
-                   double2* zbuf, int rows_per_pass, double* out_re, double* out_im, cudaStream_t st, int npieces, float2* Kff) {
+                   double2* zbuf, int rows_per_pass, double* out_re, double* out_im, cudaStream_t st, int npieces, float2* Kff,
+                   unsigned char* redo) {
     const long long tot = (long long)d.U * (nk + nq);
     const size_t es = precision == SGL_FP64 ? 8 : 4;
     void* e = tables;
@@ -1197,10 +1216,11 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
             SGL_COUNT(1);
         } else if (Kff) {
             k_vp_chain_ff<<<ceil_div(NP, kCfPts), kCfThreads, sizeof(ChainShared), st>>>(d, Kff, zp, al, NP, nq, kb, out_re,
-                                                                                         out_im, npieces);
-            SGL_COUNT(1);
+                                                                                         out_im, npieces, redo);
+            k_vp_chain<<<ceil_div(NP, kChPts), kChPts, chain_smem, st>>>(d, zp, al, NP, nq, kb, out_re, out_im, npieces, redo);
+            SGL_COUNT(2);
         } else {
-            k_vp_chain<<<ceil_div(NP, kChPts), kChPts, chain_smem, st>>>(d, zp, al, NP, nq, kb, out_re, out_im, npieces);
+            k_vp_chain<<<ceil_div(NP, kChPts), kChPts, chain_smem, st>>>(d, zp, al, NP, nq, kb, out_re, out_im, npieces, nullptr);
             SGL_COUNT(1);
         }
     }
