@@ -257,8 +257,8 @@ k_vp_z(VpDevice d, const typename V2<TT>::T* __restrict__ e, const typename V2<T
 constexpr int kZlThreads = 128;
 
 __global__ void __launch_bounds__(kZlThreads)
-k_vp_z_line(VpDevice d, const float2* __restrict__ e, const float2* __restrict__ Jt, int nk, int nq, double2* __restrict__ zp,
-            double2* __restrict__ alin, long long NP, int npieces) {
+k_vp_z_line(VpDevice d, const float2* __restrict__ e, const float2* __restrict__ Jt, int nk, int nq, int kb,
+            double2* __restrict__ zp, double2* __restrict__ alin, long long NP, int npieces) {
     const int lane = threadIdx.x & 31, g = blockIdx.y * (kZlThreads / 32) + (threadIdx.x >> 5);
     if (g >= d.nsh * npieces) return;
     const int s = g / npieces, piece = g % npieces;
@@ -267,7 +267,7 @@ k_vp_z_line(VpDevice d, const float2* __restrict__ e, const float2* __restrict__
     const long long p = (long long)blockIdx.x * 32 + lane;
     const bool live = p < NP;
     const int pp = live ? (int)p : 0;
-    const float2* ek = e + pp / nq;
+    const float2* ek = e + kb + pp / nq;                     // kb: first row of the pass
     const float2* jq = Jt + pp % nq;
     double SAr = 0.0, SAi = 0.0, SBr = 0.0, SBi = 0.0, ALr = 0.0, ALi = 0.0;
     int jcur = 0;
@@ -1199,7 +1199,7 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
             SGL_COUNT(1);
         } else if (vp_line(precision, nk, nq)) {
             const dim3 gl(ceil_div(NP, 32), ceil_div((long long)d.nsh * npieces, kZlThreads / 32));
-            k_vp_z_line<<<gl, kZlThreads, 0, st>>>(d, (const float2*)e, (const float2*)Jt, nk, nq, zp, al, NP, npieces);
+            k_vp_z_line<<<gl, kZlThreads, 0, st>>>(d, (const float2*)e, (const float2*)Jt, nk, nq, kb, zp, al, NP, npieces);
             SGL_COUNT(1);
         } else {
             k_vp_z<float><<<g1, kZThreads, 0, st>>>(d, (const float2*)e, (const float2*)Jt, nk, nq, kb, nkc, zp, al, NP,
