@@ -297,7 +297,8 @@ sgl_status sgl_batch_pdf(sgl_batch* batch, int n_jobs, const int32_t* job_slot, 
  * item and every resident CTA).  A batch that was not tuned takes 64 k-points per item and every
  * resident CTA.
  * sgl_cfb_lnphi runs the persistent solve (CTAs take (instance, k tile, part of a gauss instance's cells) items from
- * a device counter, longest instances first; parts are summed in order) and copies ln Phi out as (re, im) pairs per k, instances in order
+ * a device counter, longest instances first; an instance's bits do not depend on the batch it is solved in) and copies
+ * ln Phi out as (re, im) pairs per k, instances in order
  * (out may be NULL).  sgl_cfb_pdf adds Phi = exp(ln Phi) and the inversion to dP/dln mu at the n_lnmu
  * points (mu = (1 - kappa)^-2): P_out is n_inst x n_lnmu; use_graph = 1 captures the whole step in a CUDA
  * graph on first use and replays it; *ms_out (may be NULL) receives the device time of the step. */

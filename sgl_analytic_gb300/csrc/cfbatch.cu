@@ -8,7 +8,9 @@
 //          latent states (weights w, transition K): the one-dimensional form of the positive Cox
 //          closure (pos_closure.py:184-240, 453-491; one group per plane).
 // Work items are (instance, tile of KT k-points, part of a gauss instance's cells), sorted by cost (longest
-// first); parts write partial sums that a second kernel adds in order (k_cfb_sum_parts).  A persistent grid
+// first).  A gauss instance is summed in segments of cells whose length follows from its own cell count
+// (cfb_segment), in order: by one item, or by items of some segments each, whose sums a second kernel adds
+// (k_cfb_sum_parts), so that its bits do not depend on the batch that it is solved in.  A persistent grid
 // of CTAs takes items from a device counter until none is left; each item stages its instance's
 // cells through shared memory (all threads of the CTA work on the same instance) and writes its
 // k-points' ln Phi.  Per-term arithmetic is that of the 1-D sweep: FP64 sincos (SGL_FP64), or the
@@ -40,9 +42,18 @@ struct CfbArgs {
     const double* vp_w;                       // [slot][nstate]
     int nstate;
     double2* out;                             // ln Phi per (instance, k)
-    double2* parts;                           // partial sums [part][instance, k] of split instances
-    long long total_k;
+    double2* parts;                           // split instances: segment sums, [segment][k] from part_off[instance]
+    const long long* part_off;
 };
+
+__device__ __forceinline__ double cfb_k(const CfbInst& I, int n) {
+    const double x = fma((double)n, I.dk, I.k0);
+    return I.geom ? exp(x) : x;
+}
+// ln Phi of a gauss instance from its sum over the cells: the clustering variance
+__device__ __forceinline__ double2 cfb_gauss(const CfbInst& I, double2 s, double k) {
+    return make_double2(fma(-0.5 * I.V * k, k, s.x), s.y);
+}
 
 // compensated sum over cells [c0, c1) for one k (thread), cells staged cooperatively
 template <int MODE, int KT>
@@ -113,22 +124,28 @@ k_cfb_persistent(CfbArgs a) {
         const CfbInst I = a.inst[wi.x];
         const int n = wi.y * KT + threadIdx.x;
         const bool live = n < I.nk;
-        auto k_at = [&](int j) { return I.geom ? exp(I.k0 + (double)j * I.dk) : I.k0 + (double)j * I.dk; };
-        const double k = live ? k_at(n) : 0.0;
+        const double k = live ? cfb_k(I, n) : 0.0;
         const CfWave kf(k);
         // the item's largest half wave number (k ascends)
-        const float khm = MODE == SGL_FP64 ? 0.f : 0.5f * (float)fmax(fabs(k_at(wi.y * KT)), fabs(k_at(min(I.nk, wi.y * KT + KT) - 1)));
+        const float khm = MODE == SGL_FP64 ? 0.f : 0.5f * (float)fmax(fabs(cfb_k(I, wi.y * KT)), fabs(cfb_k(I, min(I.nk, wi.y * KT + KT) - 1)));
         double2 lp;
         if (I.closure == 0) {
-            // parts are whole tiles of cells
-            const long long per = ((I.c1 - I.c0 + wi.w - 1) / wi.w + kCfbTile - 1) / kCfbTile * kCfbTile;
-            const long long c0 = min(I.c1, I.c0 + wi.z * per);
-            const double2 s = cfb_cells<MODE, KT>(a, c0, min(I.c1, c0 + per), k, kf, khm, s_f, s_k, s_w);
-            if (wi.w > 1) {
-                if (live) a.parts[wi.z * a.total_k + I.k_off + n] = s;
-                continue;
+            const long long seg = cfb_segment(I.c1 - I.c0), ns = (I.c1 - I.c0 + seg - 1) / seg;
+            const long long q0 = ns * wi.z / wi.w, q1 = ns * (wi.z + 1) / wi.w;
+            double2* part = wi.w > 1 ? a.parts + a.part_off[wi.x] + n : nullptr;
+            double2 s = make_double2(0.0, 0.0);
+            for (long long q = q0; q < q1; ++q) {
+                const long long c0 = I.c0 + q * seg;
+                const double2 v = cfb_cells<MODE, KT>(a, c0, min(I.c1, c0 + seg), k, kf, khm, s_f, s_k, s_w);
+                if (part) {
+                    if (live) part[q * I.nk] = v;
+                } else {
+                    s.x += v.x;
+                    s.y += v.y;
+                }
             }
-            lp = make_double2(s.x - 0.5 * I.V * k * k, s.y);
+            if (part) continue;
+            lp = cfb_gauss(I, s, k);
         } else if (MODE == SGL_FP64) {
             // Poisson sum plus the chain: alpha_t = (sum_s alpha_s K_st) e^{z_t}, z_t = D_pt Lambda_p,
             // rescaled by its largest modulus each plane (the scale kept as a logarithm)
@@ -267,24 +284,25 @@ __device__ __forceinline__ int cfb_inst_of(const long long* k_offs, int n_inst, 
     return lo;
 }
 
-// ln Phi of the split instances: their parts' sums in order, and the clustering variance
+// ln Phi of the split instances: their segments' sums in order, and the clustering variance
 __global__ void k_cfb_sum_parts(const CfbInst* __restrict__ inst, int n_inst, const long long* __restrict__ k_offs,
-                                const int* __restrict__ nparts, const double2* __restrict__ parts, long long total,
+                                const long long* __restrict__ part_off, const double2* __restrict__ parts, long long total,
                                 double2* __restrict__ out) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
     const int i = cfb_inst_of(k_offs, n_inst, e);
-    const int np = nparts[i];
-    if (np <= 1) return;
+    if (part_off[i] < 0) return;                      // not split
     const CfbInst I = inst[i];
-    double sr = 0.0, si = 0.0;
-    for (int p = 0; p < np; ++p) {
-        const double2 v = parts[p * total + e];
-        sr += v.x;
-        si += v.y;
+    const long long seg = cfb_segment(I.c1 - I.c0), ns = (I.c1 - I.c0 + seg - 1) / seg;
+    const int n = (int)(e - I.k_off);
+    const double2* p = parts + part_off[i] + n;
+    double2 s = make_double2(0.0, 0.0);
+    for (long long q = 0; q < ns; ++q) {
+        const double2 v = p[q * I.nk];
+        s.x += v.x;
+        s.y += v.y;
     }
-    const double x = I.k0 + (double)(e - I.k_off) * I.dk, k = I.geom ? exp(x) : x;
-    out[e] = make_double2(sr - 0.5 * I.V * k * k, si);
+    out[e] = cfb_gauss(I, s, cfb_k(I, n));
 }
 
 // Phi(k_n) w_n / pi (trapezoid weights) per (instance, k), FP64 or FP32 planes
@@ -404,8 +422,8 @@ void launch_cfb_persistent(int precision, int kt, int ctas, const CfbInst* inst,
                            int* counter, const long long* plane_cells, const double* kap, const double* w,
                            const float* kh, const float* kl, const float* wf, const double* vp_D, const double* vp_K,
                            const double* vp_w, int nstate, double2* out, cudaStream_t st, double2* parts, int n_inst,
-                           const long long* k_offs, const int* nparts, long long total_k) {
-    CfbArgs a{inst, items, n_items, counter, plane_cells, kap, w, kh, kl, wf, vp_D, vp_K, vp_w, nstate, out, parts, total_k};
+                           const long long* k_offs, const long long* part_off, long long total_k) {
+    CfbArgs a{inst, items, n_items, counter, plane_cells, kap, w, kh, kl, wf, vp_D, vp_K, vp_w, nstate, out, parts, part_off};
     cudaMemsetAsync(counter, 0, sizeof(int), st);
 #define SGL_CFB_LAUNCH(M, T) k_cfb_persistent<M, T><<<ctas, T, 0, st>>>(a)
     if (precision == SGL_FP64) {
@@ -416,7 +434,7 @@ void launch_cfb_persistent(int precision, int kt, int ctas, const CfbInst* inst,
 #undef SGL_CFB_LAUNCH
     SGL_COUNT(1);
     if (parts) {
-        k_cfb_sum_parts<<<ceil_div(total_k, 256), 256, 0, st>>>(inst, n_inst, k_offs, nparts, parts, total_k, out);
+        k_cfb_sum_parts<<<ceil_div(total_k, 256), 256, 0, st>>>(inst, n_inst, k_offs, part_off, parts, total_k, out);
         SGL_COUNT(1);
     }
 }

@@ -60,16 +60,32 @@ std::vector<int4> cfb_items(const CfbState& S, int kt, const std::vector<int>& o
 
 // The parts of each gauss instance's cells: a batch with few (instance, k tile) pairs (planes solved at 128 nodes each)
 // would leave CTAs idle or one item running alone at the end, so its items are cut into about four per resident
-// CTA, of at least four tiles of 512 cells.  6 x 64 planes of 131072 cells at 128 nodes: solve 10.6 -> 6.0 ms.
-std::vector<int> cfb_nparts(const CfbState& S, int kt, int ctas, int* most) {
+// CTA, of whole segments (cfb_segment).  6 x 64 planes of 131072 cells at 128 nodes: solve 10.6 -> 6.0 ms.  part_off: where
+// a split instance's segment sums start, -1 where it is not split; *elems of them in all.  Nothing is split when they would
+// take more than kCfbPartBytes.
+constexpr long long kCfbPartBytes = 1LL << 30;
+
+std::vector<int> cfb_nparts(const CfbState& S, int kt, int ctas, std::vector<long long>* part_off, long long* elems) {
     long long tiles = 0;
     for (const CfbInst& I : S.inst) tiles += (I.nk + kt - 1) / kt;
     const long long want = std::min<long long>(64, (4LL * ctas + tiles - 1) / tiles);
-    *most = 1;
     std::vector<int> np(S.inst.size(), 1);
-    for (size_t i = 0; i < S.inst.size(); ++i)
-        if (S.inst[i].closure == 0)
-            *most = std::max(*most, np[i] = (int)std::max<long long>(1, std::min(want, (S.inst[i].c1 - S.inst[i].c0) / 2048)));
+    part_off->assign(S.inst.size(), -1);
+    *elems = 0;
+    for (size_t i = 0; i < S.inst.size(); ++i) {
+        const CfbInst& I = S.inst[i];
+        const long long cells = I.c1 - I.c0, seg = cfb_segment(cells);
+        if (I.closure == 0) np[i] = (int)std::max<long long>(1, std::min(want, cells / seg));
+        if (np[i] > 1) {
+            (*part_off)[i] = *elems;
+            *elems += (cells + seg - 1) / seg * I.nk;
+        }
+    }
+    if (*elems * 16 > kCfbPartBytes) {
+        np.assign(np.size(), 1);
+        part_off->assign(part_off->size(), -1);
+        *elems = 0;
+    }
     return np;
 }
 
@@ -79,7 +95,7 @@ struct CfbRun {
     int n_items = 0, ctas = 0, kt = 0;
     int* counter = nullptr;
     double2* lnphi = nullptr; double2* parts = nullptr;
-    int* nparts = nullptr;
+    long long* part_off = nullptr;
 };
 
 sgl_status cfb_prepare(sgl_ctx* ctx, int precision, int kt, int cps, const std::vector<int4>* given, const std::string& tag,
@@ -90,11 +106,11 @@ sgl_status cfb_prepare(sgl_ctx* ctx, int precision, int kt, int cps, const std::
     if (res < 1) return fail(ctx, SGL_ERR_CUDA, "batched CF kernel: no resident CTA for this tile width");
     R.kt = kt;
     R.ctas = kNumSMs * std::max(1, std::min(cps, res));
-    int most = 1;
+    long long part_elems = 0;
     std::vector<int4> own;
-    std::vector<int> np;
+    std::vector<long long> part_off;
     if (!given) {
-        np = cfb_nparts(S, kt, R.ctas, &most);
+        const std::vector<int> np = cfb_nparts(S, kt, R.ctas, &part_off, &part_elems);
         own = cfb_items(S, kt, S.order, np);
         given = &own;
     }
@@ -105,11 +121,11 @@ sgl_status cfb_prepare(sgl_ctx* ctx, int precision, int kt, int cps, const std::
     R.lnphi = dbuf<double2>(ctx, "cfb_lnphi", (size_t)std::max<long long>(1, S.total_k));
     if (!R.items || !R.counter || !R.lnphi) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (batched CF solve)");
     CKS(upload(ctx, R.items, given->data(), given->size()));
-    if (most > 1) {
-        R.parts = dbuf<double2>(ctx, "cfb_parts_" + tag, (size_t)most * S.total_k);
-        R.nparts = dbuf<int>(ctx, "cfb_nparts_" + tag, np.size());
-        if (!R.parts || !R.nparts) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (batched CF solve)");
-        CKS(upload(ctx, R.nparts, np.data(), np.size()));
+    if (part_elems > 0) {
+        R.parts = dbuf<double2>(ctx, "cfb_parts_" + tag, (size_t)part_elems);
+        R.part_off = dbuf<long long>(ctx, "cfb_part_off_" + tag, part_off.size());
+        if (!R.parts || !R.part_off) return fail(ctx, SGL_ERR_CUDA, "device allocation failed (batched CF solve)");
+        CKS(upload(ctx, R.part_off, part_off.data(), part_off.size()));
     }
     if (!S.have[P]) {
         // template planes: the cells in this precision's form
@@ -142,7 +158,7 @@ void cfb_enqueue(sgl_ctx* ctx, int precision, const CfbRun& R) {
                           (const float*)ctx->arena.find("cfb_wf"), (const double*)ctx->arena.find("cfb_vpD"),
                           (const double*)ctx->arena.find("cfb_vpK"), (const double*)ctx->arena.find("cfb_vpw"),
                           S.nstate, R.lnphi, ctx->stream, R.parts, S.n_inst,
-                          (const long long*)ctx->arena.find("cfb_koffs"), R.nparts, S.total_k);
+                          (const long long*)ctx->arena.find("cfb_koffs"), R.part_off, S.total_k);
 }
 
 sgl_status cfb_launch(sgl_ctx* ctx, int precision, int kt, int cps, const std::vector<int4>* items,

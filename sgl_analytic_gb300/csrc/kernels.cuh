@@ -147,12 +147,17 @@ struct CfbInst {                          // one instance of the batch
     int geom;                             // 1: the solve's k points are exp(k0 + n dk) (log-spaced)
     double k0;                            // else k0 + n dk (the inversion assumes k0 = 0)
 };
-// items (instance, k tile, part, parts); parts buffer and nparts per instance only when some instance is split
+// a gauss instance's cells are summed in segments of this length (whole tiles of 512; at most 64 segments)
+__host__ __device__ constexpr long long cfb_segment(long long cells) {
+    return cells <= 64 * 2048 ? 2048 : (cells + 64 * 512 - 1) / (64 * 512) * 512;
+}
+// items (instance, k tile, part, parts); parts, with the start of each split instance's segment sums (< 0: not split), only
+// when some instance is split
 void launch_cfb_persistent(int precision, int kt, int ctas, const CfbInst* inst, const int4* items, int n_items,
                            int* counter, const long long* plane_cells, const double* kap, const double* w,
                            const float* kh, const float* kl, const float* wf, const double* vp_D, const double* vp_K,
                            const double* vp_w, int nstate, double2* out, cudaStream_t st, double2* parts, int n_inst,
-                           const long long* k_offs, const int* nparts, long long total_k);
+                           const long long* k_offs, const long long* part_off, long long total_k);
 void launch_cfb_pdf(int precision, const CfbInst* inst, int n_inst, const double2* lnphi, long long total,
                     const long long* k_offs, void* phi, const double* lnmu, int nm, double* P, cudaStream_t st);
 int cfb_resident_ctas(int precision, int kt);
