@@ -556,6 +556,8 @@ sgl_status sep_gemms(sgl_ctx* ctx, int precision, const double* h_kg, const doub
 //   xi term: 101^2 coarse grid + not-a-knot bicubic spline when the grid has more than 101^2
 //   points (and both axes > 1 point, both maxima > 0), exact otherwise.
 // write_phi = 1 writes Phi = exp(ln Phi) in the precision's element type (inversion path).
+constexpr int kHalfAngleCells = 1 << 21;
+
 sgl_status lambda_eval(sgl_ctx* ctx, int precision, const double* h_kk, int nk, const double* h_kg, int nkg,
                        int write_phi, void* out_re, void* out_im) {
     cudaStream_t st = ctx->stream;
@@ -668,10 +670,11 @@ sgl_status lambda_eval(sgl_ctx* ctx, int precision, const double* h_kk, int nk, 
             Timed t(ctx, precision == SGL_FP64 ? "sep_sweep_f64" : "sep_sweep_mixed", (double)nk * ctx->sep.n_cells,
                     (double)ctx->sep.n_cols * ld * es);
             // FP64 rows k_n = k_0 + n dk >= 0 up to their rounding (the inversion's linspace) take the uniform sweep;
-            // two table entries of 16 B per row and cell pay from about one warp of rows on
+            // 32 table entries of 16 B per cell pay from about one warp of rows on; a table of more than 1 GiB (2^21 cells)
+            // is not built
             double dk = 0.0;
             double2* tab = nullptr;
-            if (precision == SGL_FP64 && nk >= 64 && ctx->sepd.n_cells < (1 << 26) && h_kk[0] >= 0.0) {
+            if (precision == SGL_FP64 && nk >= 64 && ctx->sepd.n_cells <= kHalfAngleCells && h_kk[0] >= 0.0) {
                 dk = (h_kk[nk - 1] - h_kk[0]) / (nk - 1);
                 bool uniform = dk > 0.0;
                 for (int i = 0; i < nk && uniform; ++i)
