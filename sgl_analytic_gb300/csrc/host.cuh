@@ -432,6 +432,21 @@ inline int* dev_err_flag(sgl_ctx* ctx) {
 // FP64 GEMMs of at least this many FLOP in all run sliced on the tensor cores (oz_gemm.cu); below, its four launches and
 // unsplit K cost more than they save (0.12 GFLOP: 0.24 ms sliced, 0.14 ms SIMT; 0.07: 0.11 and 0.07; 6.9: 0.52 and 5.8)
 constexpr double kOzMinFlops = 4e8;
+
+// ... unless a few tiles with a long K would leave the chip idle, K being unsplit: a 128 x 64 tile takes 57 ns per k, the
+// launches 0.08 ms, and the SIMT kernel (K in slices) 1.15 TFLOP/s on 64 x 64 tiles.  M x N x K, sliced / SIMT in ms:
+// 128 x 64 x 60000 3.4 / 1.15, 256 x 64 x 16000 0.99 / 0.48, 60 x 500 x 8000 0.55 / 0.46, 200 x 100 x 10000 0.64 / 0.61;
+// 120 x 500 x 4000 0.30 / 0.45, 400 x 500 x 1000 0.13 / 0.40, 1000 x 102 x 2000 0.22 / 0.39.
+inline bool oz_pays(const std::vector<GemmDesc<double>>& d) {
+    double fl = 0.0, load = 0.0, longest = 0.0, simt = 0.0;
+    for (const auto& g : d) {
+        fl += 2.0 * g.M * (double)g.N * g.K;
+        simt += 2.0 * 64 * ceil_div(g.M, 64) * (64.0 * ceil_div(g.N, 64)) * g.K;
+        load += (double)ceil_div(g.M, 128) * ceil_div(g.N, 64) * g.K;
+        longest = std::max(longest, (double)g.K);
+    }
+    return fl >= kOzMinFlops && 57e-9 * std::max(longest, load / kNumSMs) + 8e-5 < simt / 1.15e12;
+}
 constexpr long long kOzBatchBytes = 1LL << 30;    // packed digits of one batch
 
 // The GEMMs of `d` in batches whose digits take at most kOzBatchBytes (a larger problem in slices of rows).  *ran = false
@@ -498,10 +513,8 @@ template <typename T>
 inline sgl_status run_gemms(sgl_ctx* ctx, std::vector<GemmDesc<T>>& d, const std::string& tag, bool fma_only = false) {
     if (d.empty()) return SGL_OK;
     if constexpr (sizeof(T) == 8) if (!fma_only) {
-        double fl = 0.0;
-        for (auto& g : d) fl += 2.0 * g.M * (double)g.N * g.K;
         bool ran = false;
-        if (fl >= kOzMinFlops) CKS(run_oz_gemms(ctx, d, tag, &ran));
+        if (oz_pays(d)) CKS(run_oz_gemms(ctx, d, tag, &ran));
         if (ran) return SGL_OK;
     }
     int tiles = gemm_plan(d.data(), (int)d.size());
@@ -582,9 +595,9 @@ GemmDesc<T> gd(int M, int N, int K, const void* A, long long ars, long long acs,
 // then a fixed-order sum (deterministic).  SIMT kernels (FP64, and FP32 where chosen below).
 template <typename T>
 inline sgl_status gemm_splitk_simt(sgl_ctx* ctx, GemmDesc<T> g, const std::string& tag, int min_split = 1) {
-    if (sizeof(T) == 8 && 2.0 * g.M * (double)g.N * g.K >= kOzMinFlops) {      // needs no K slices
+    if constexpr (sizeof(T) == 8) {
         std::vector<GemmDesc<T>> v{g};
-        return run_gemms(ctx, v, tag);
+        if (oz_pays(v)) return run_gemms(ctx, v, tag);                          // needs no K slices
     }
     GemmDesc<T> tmp = g;
     const int tiles = gemm_plan(&tmp, 1);
