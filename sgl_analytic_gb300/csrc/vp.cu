@@ -1106,8 +1106,10 @@ k_vp_chain_small(VpDevice d, const double2* __restrict__ zp, const double2* __re
     }
 }
 
-// the mixed path's grid kernel pays from a few tiles of points on
-bool vp_mixed_grid(int precision, int nk, int nq) { return precision != SGL_FP64 && nk >= 8 && nq >= 32; }
+// The mixed path's grid kernel works on 112 columns at a time, k_vp_z on 32, at 0.4 of its time per column: up to 32 columns
+// k_vp_z is the faster one.  ln R on 6 shells, 193 k cells, grid kernel / k_vp_z in ms: 409 x 32 4.44 / 3.66, 409 x 33 4.43 /
+// 5.04, 409 x 113 7.46 / 8.40, 8 x 33 0.80 / 0.87, 16 x 40 0.98 / 1.37
+bool vp_mixed_grid(int precision, int nk, int nq) { return precision != SGL_FP64 && nk >= 8 && nq > 32; }
 static int vp_nqp(int nq) { return ceil_div(nq, kMzQ) * kMzQ; }
 
 size_t vp_table_bytes(int precision, int U, int nk, int nq, int nruns) {
