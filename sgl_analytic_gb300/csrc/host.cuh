@@ -606,7 +606,7 @@ inline sgl_status gemm_splitk_simt(sgl_ctx* ctx, GemmDesc<T> g, const std::strin
     // min_split > 1 (mixed path): at least min_split slices of at least 32 terms; FP32 slices
     // are combined in float-float
     split = std::max(split, std::min(min_split, std::max(1, g.K / 32)));
-    if (split <= 1) { std::vector<GemmDesc<T>> v{g}; return run_gemms(ctx, v, tag); }
+    if (split <= 1) { std::vector<GemmDesc<T>> v{g}; return run_gemms(ctx, v, tag, true); }
     const long long slice = (long long)g.M * g.N;
     DBUF(ws, T, "splitk_ws_" + tag, slice * split);
     std::vector<GemmDesc<T>> v;
@@ -623,7 +623,7 @@ inline sgl_status gemm_splitk_simt(sgl_ctx* ctx, GemmDesc<T> g, const std::strin
         p.beta = T(0);
         v.push_back(p);
     }
-    CKS(run_gemms(ctx, v, tag));
+    CKS(run_gemms(ctx, v, tag, true));
     launch_sum_slices<T>(ws, (int)v.size(), g.M, g.N, g.C, g.ldc, g.beta, ctx->stream);
     CKLAUNCH();
     return SGL_OK;
