@@ -296,7 +296,7 @@ sgl_status sgl_sweep_eval(sgl_ctx* ctx, const double* kk, int nk, int precision,
     for (int i = 0; i < nk; ++i) if (!std::isfinite(kk[i])) return fail(ctx, SGL_ERR_VALUE, "non-finite kk");
     CK(cudaSetDevice(ctx->device));
     const long long nc = ctx->sweep_n;
-    const int nch = sweep1d_chunks(nk, nc);
+    const int nch = sweep1d_chunks(precision, nk, nc);
     DBUF(d_kk, double, "sw_kk", nk);
     DBUF(d_part, double2, "sw_part", (long long)nch * nk);
     DBUF(d_out, double, "sw_out", 2LL * nk);

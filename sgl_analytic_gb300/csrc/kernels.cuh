@@ -329,7 +329,7 @@ void launch_vp_lnR(int precision, const VpDevice& d, const double* kv, int nk, c
 int vp_pieces(int precision, int nsh, int rows, int nq);
 
 // ---- 1-D CF sweep and FMA probes
-int sweep1d_chunks(int nk, long long nc);
+int sweep1d_chunks(int precision, int nk, long long nc);
 void launch_sweep1d(int precision, const double* kk, int nk, const double* kap, const double* w, const float* kh,
                     const float* kl, const float* wf, long long nc, int nchunks, double2* part, double* re,
                     double* im, cudaStream_t st);

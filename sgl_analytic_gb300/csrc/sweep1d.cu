@@ -10,6 +10,8 @@
 // terms/s) with the packed terms.
 //
 // Also: FMA-throughput probes used as the measured FP64 / FP32 peaks of the CF-sweep roofline.
+#include <algorithm>
+
 #include "cfterm.cuh"
 #include "kernels.cuh"
 
@@ -93,14 +95,17 @@ __global__ void k_sweep1d_reduce(const double2* __restrict__ part, int nchunks, 
     im[n] = i;
 }
 
-int sweep1d_chunks(int nk, long long nc) {
-    // 32 CTAs per SM over (k tiles x chunks): about 8 waves of 4 resident CTAs, so that the last, partly filled
-    // wave costs little; no chunk below 4 tiles of cells
-    const int ktiles = ceil_div(nk, kSwRows);
-    long long nch = (32LL * kNumSMs + ktiles - 1) / ktiles;
-    const long long maxch = (nc + 4 * kSwTile - 1) / (4 * kSwTile);
-    if (nch > maxch) nch = maxch;
-    return (int)(nch < 1 ? 1 : nch);
+int sweep1d_chunks(int precision, int nk, long long nc) {
+    // At least 4 CTAs per SM over (k tiles x chunks), down to chunks of one tile of cells: few cells at few k need every
+    // CTA (FP64, 16384 cells x 100 k: 32 chunks of a tile 3.1 ms, 8 of four 12.2).  Mixed: up to 32 CTAs per SM, about 8
+    // waves of 4 resident CTAs, so that the last, partly filled wave costs little, of no less than 4 tiles.
+    const long long ktiles = ceil_div(nk, kSwRows);
+    auto chunks = [&](long long per_sm, long long tiles) {
+        return std::min((per_sm * kNumSMs + ktiles - 1) / ktiles, (nc + tiles * kSwTile - 1) / (tiles * kSwTile));
+    };
+    long long nch = chunks(4, 1);
+    if (precision != SGL_FP64) nch = std::max(nch, chunks(32, 4));
+    return (int)std::max(1LL, nch);
 }
 
 void launch_sweep1d(int precision, const double* kk, int nk, const double* kap, const double* w, const float* kh,
