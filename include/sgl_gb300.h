@@ -295,7 +295,7 @@ sgl_status sgl_batch_pdf(sgl_batch* batch, int n_jobs, const int32_t* job_slot, 
  * SM) shape on a work-bounded sample of the batch and keeps the fastest for the context's batches of its shape
  * class (largest k grid and mean cells per instance, in powers of two; SGL_MIXED: SGL_FP64 takes 128 k-points per
  * item and every resident CTA).  A batch that was not tuned takes 64 k-points per item and every
- * resident CTA.
+ * resident CTA, or as many as share its vp instances' items evenly where these do not fill the chip.
  * sgl_cfb_lnphi runs the persistent solve (CTAs take (instance, k tile, part of a gauss instance's cells) items from
  * a device counter, longest instances first; an instance's bits do not depend on the batch it is solved in) and copies
  * ln Phi out as (re, im) pairs per k, instances in order

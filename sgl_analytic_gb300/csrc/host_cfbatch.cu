@@ -170,14 +170,24 @@ sgl_status cfb_launch(sgl_ctx* ctx, int precision, int kt, int cps, const std::v
     return SGL_OK;
 }
 
-// The launch shape used when none was tuned: every resident CTA, 64 k-points per item in mixed precision (two warps wait
-// at the barriers of a plane's few cells; 41 gauss and vp instances: step 19.4 ms, 128 wide 19.6; planes at 128 nodes
-// the same within 2%), 128 in FP64.  Timing all shapes on first use, as this did, cost 0.6 s per context.
+// The launch shape used when none was tuned: 64 k-points per item in mixed precision (two warps wait at the barriers of a
+// plane's few cells; 41 gauss and vp instances: step 19.4 ms, 128 wide 19.6; planes at 128 nodes the same within 2%), 128
+// in FP64, and every resident CTA.  Timing all shapes on first use, as this did, cost 0.6 s per context.
+// The items of a vp instance are not split and come first; where they do not fill the chip, as many CTAs per SM as share
+// them evenly (at least 3, for the gauss items beside them), because more of them meet on some SMs and set the time.  CTAs
+// per SM -> step in ms, mixed: 420 vp items 2: 3.70, 3: 2.29, 4: 2.56, 8: 3.91, all (16): 3.90; 248 items 2: 1.63, 3: 1.41,
+// all 1.82; 760 items 4: 3.02, 5: 3.34, all 4.25; 908 items 6: 4.82, all 5.14; 1728 items 8 and more: 4.85.
 void cfb_default_shape(sgl_ctx* ctx, int precision) {
     CfbState& S = *ctx->cfb;
     const int P = precision == SGL_FP64 ? 0 : 1;
     S.kt[P] = P == 1 ? 64 : 128;
     S.cps[P] = std::max(1, cfb_resident_ctas(precision, S.kt[P]));
+    if (P == 1) {
+        long long vp = 0;
+        for (const CfbInst& I : S.inst)
+            if (I.closure == 1) vp += (I.nk + S.kt[P] - 1) / S.kt[P];
+        if (vp > 0) S.cps[P] = (int)std::min<long long>(S.cps[P], std::max<long long>(3, (vp + kNumSMs - 1) / kNumSMs));
+    }
     S.tuned[P] = true;
 }
 
