@@ -258,7 +258,7 @@ void launch_mlp_fused(int n, const float* X, const float* const* W_dev, const fl
                       float* small, const float** ptrs, float* Y, int* err, int ctas, cudaStream_t st);
 void launch_bias_act(int M, int N, const float* Z, const float* bias, float* Zb, float* A, int silu, cudaStream_t st);
 void launch_act_grad(int M, int N, const float* dA, const float* Zb, float* dZ, cudaStream_t st);
-long long col_sum_parts(int M, int N);   // doubles of scratch
+long long col_sum_parts(int M, int N);   // doubles of scratch (0: none)
 void launch_col_sum(int M, int N, const float* X, double* part, float* out, cudaStream_t st);
 int mse_blocks(long long n);
 void launch_mse(long long n, const float* pred, const float* tgt, float* dpred, double* part, cudaStream_t st);

@@ -25,9 +25,11 @@ __global__ void k_act_grad(int M, int N, const float* __restrict__ dA, const flo
     dZ[e] = dA[e] * sg * (1.f + z * (1.f - sg));
 }
 
-// out[j] = sum_i X[i, j] in FP64: a CTA per (128 columns, 64 rows) adds its rows column by column (coalesced), a second
-// pass adds the CTAs' sums in order.  One CTA per column, 4-byte reads N apart, took 45 us for 16384 x 256; this, 26.
-constexpr int kColRows = 64;
+// out[j] = sum_i X[i, j] in FP64.  Up to kColDirect rows: one CTA per column, its reads N apart but in L2 (the operand was
+// just written).  Above: a CTA per (128 columns, 64 rows) adds its rows column by column (coalesced), and a second pass the
+// CTAs' sums in order.  Per call, direct / two passes in us: 64 x 256 4.6 / 12.8, 4096 x 256 10.6 / 14.0, 16384 x 256 23 / 28,
+// 20 x 5000 19 / 25, 100000 x 256 259 / 111, 300000 x 8 269 / 59, 1000000 x 2 854 / 147.
+constexpr int kColRows = 64, kColDirect = 1 << 15;
 __global__ void __launch_bounds__(128) k_col_part(int M, int N, int rows, const float* __restrict__ X, double* __restrict__ part) {
     const int j = blockIdx.x * 128 + threadIdx.x;
     if (j >= N) return;
@@ -43,11 +45,12 @@ __global__ void __launch_bounds__(128) k_col_part(int M, int N, int rows, const 
     part[(long long)blockIdx.y * N + j] = a0 + a1;
 }
 
-__global__ void __launch_bounds__(256) k_col_sum(int np, int N, const double* __restrict__ part, float* __restrict__ out) {
+template <typename T>
+__global__ void __launch_bounds__(256) k_col_sum(int M, int N, const T* __restrict__ X, float* __restrict__ out) {
     __shared__ double sh[32];
     const int j = blockIdx.x;
     double a = 0.0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) a += part[(long long)i * N + j];
+    for (int i = threadIdx.x; i < M; i += blockDim.x) a += (double)X[(long long)i * N + j];
     a = block_sum(a, sh);
     if (threadIdx.x == 0) out[j] = (float)a;
 }
@@ -87,14 +90,15 @@ void launch_act_grad(int M, int N, const float* dA, const float* Zb, float* dZ, 
     const long long t = (long long)M * N;
     if (t > 0) { k_act_grad<<<ceil_div(t, 256), 256, 0, st>>>(M, N, dA, Zb, dZ); SGL_COUNT(1); }
 }
-int col_sum_rows(int M) { return std::max(kColRows, ceil_div(M, 65535)); }      // rows per CTA: grid.y <= 65535
-long long col_sum_parts(int M, int N) { return (long long)std::max(1, ceil_div(M, col_sum_rows(M))) * N; }
+static int col_sum_rows(int M) { return std::max(kColRows, ceil_div(M, 65535)); }      // rows per CTA: grid.y <= 65535
+long long col_sum_parts(int M, int N) { return M <= kColDirect ? 0 : (long long)ceil_div(M, col_sum_rows(M)) * N; }
 void launch_col_sum(int M, int N, const float* X, double* part, float* out, cudaStream_t st) {
     if (N <= 0) return;
+    if (M <= kColDirect) { k_col_sum<<<N, 256, 0, st>>>(M, N, X, out); SGL_COUNT(1); return; }
     const int rows = col_sum_rows(M), np = ceil_div(M, rows);
-    if (np > 0) { k_col_part<<<dim3(ceil_div(N, 128), np), 128, 0, st>>>(M, N, rows, X, part); SGL_COUNT(1); }
+    k_col_part<<<dim3(ceil_div(N, 128), np), 128, 0, st>>>(M, N, rows, X, part);
     k_col_sum<<<N, 256, 0, st>>>(np, N, part, out);
-    SGL_COUNT(1);
+    SGL_COUNT(2);
 }
 int mse_blocks(long long n) { return (int)std::min<long long>(1024, std::max<long long>(1, ceil_div(n, 256))); }
 void launch_mse(long long n, const float* pred, const float* tgt, float* dpred, double* part, cudaStream_t st) {
