@@ -98,17 +98,21 @@ k_tc_pack_bf16(const TcPackDesc* __restrict__ descs, int nprob, float* __restric
     const int lane = (int)(q & 31), c = lane >> 3;
     const int r = (int)(grp % (d.Rpad >> 3)) * 8 + (lane & 7), kb = (int)(grp / (d.Rpad >> 3));
     uint32_t w[4];
-    auto element = [&](int k) {
-        if (r >= d.R || k >= d.K) return 0.f;
-        const bool low = d.fold > 0 && k >= d.fold;
-        const float v = __ldg(d.X + (long long)r * d.x_rs + (long long)(low ? k - d.fold : k) * d.x_cs);
-        return low && d.part ? v - __bfloat162float(__float2bfloat16_rn(v)) : v;
-    };
+    float v[8];
+    const int k0 = kb * 32 + c * 8;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {                        // the eight loads in flight together
+        const int k = k0 + e, kk = d.fold > 0 && k >= d.fold ? k - d.fold : k;
+        v[e] = r < d.R && k < d.K ? __ldg(d.X + (long long)r * d.x_rs + (long long)kk * d.x_cs) : 0.f;
+    }
+    if (d.fold > 0 && d.part) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (k0 + e >= d.fold) v[e] -= __bfloat162float(__float2bfloat16_rn(v[e]));
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        const int k = kb * 32 + c * 8 + 2 * e;
-        const float v0 = element(k), v1 = element(k + 1);
-        const __nv_bfloat162 b2 = __floats2bfloat162_rn(v0, v1);
+        const __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
         w[e] = *(const uint32_t*)&b2;
     }
     unsigned char* out = (unsigned char*)(base + d.out_off);
