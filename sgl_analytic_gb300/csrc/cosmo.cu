@@ -257,7 +257,8 @@ __global__ void __launch_bounds__(kPartThreads) k_cos_parts(CosArgs a) {
     }
 }
 
-// 1 / d for 1 <= d < 1e300: PTX's approximate reciprocal (relative error below 2^-23) and two Newton steps
+// 1 / d for 1 <= d < 1e300: PTX's approximate reciprocal (the operand's upper 32 bits, a 20-bit mantissa: relative error
+// below 2^-19) and two Newton steps (2^-38, then FP64's own rounding)
 __device__ __forceinline__ double recip(double d) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));

@@ -147,8 +147,10 @@ sgl_status sgl_gemm_bf16(sgl_ctx* ctx, int M, int N, int K, const float* A, int6
     t.C = C; t.c_rs = c_rs; t.c_cs = c_cs;
     t.alpha = alpha;
     // few tiles and a long K (a weight gradient: K = the batch): columns in tiles of 32, so that more CTAs load and
-    // multiply (256 x 256 x 16384: 203 -> 139 us; 16 and 64 columns the same).  K is not sliced: TMEM sums truncate, and a gradient whose terms cancel moves
-    // by the truncation that slicing removes (1.4e-5 of it as a rule, 3.6e-4 on one batch in a hundred).
+    // multiply.  Calls in a row, 256 / 32 columns in us: 256 x 256 x 4096 57.3 / 55.8, x 16384 162 / 160, x 65536 635 / 593,
+    // 300 x 300 x 9000 101 / 99, 2048 x 256 x 4096 63.9 / 63.3 (16 and 64 columns the same): a chain of K blocks bounds
+    // them.  K is not sliced: TMEM sums truncate, and a gradient whose terms cancel moves by the truncation that slicing
+    // removes (1.4e-5 of it as a rule, 3.6e-4 on one batch in a hundred).
     const bool thin = K >= 4096 && ceil_div(M, 128) * ceil_div(N, 256) <= 16;
     return run_tc_gemms(ctx, v, "bf16", 1, false, thin ? 32 : 256);
 }

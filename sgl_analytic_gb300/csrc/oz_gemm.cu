@@ -7,16 +7,20 @@
 //   A(i, k) = 2^(ea_i - 55) sum_s a_s(i, k) 256^(6 - s),   s = 0 .. 6,
 // the largest element of a row exactly, smaller ones to 2^-56 of it.  Before that, column k of A is divided and row k of
 // B multiplied by the power of two of the column's largest element: where large elements of A meet small ones of B (the
-// separable expansion's weights against J0 - 1) the scales then follow the products.  The digit products of equal weight,
+// separable expansion's weights against J0 - 1) the scales then follow the products; an empty column takes its row of B
+// out of the scales.  The digit products of equal weight,
 // D_d = sum_k sum_{s + t = d} a_s b_t, d = 0 .. 6, are formed by tcgen05.mma.kind::f16 in FP32 accumulators: over
 // kOzDrainK = 128 k and at most 7 digit pairs every partial sum is an integer of at most 128 * 7 * 2^14 < 2^24, so no
 // accumulation rounds.  Every 128 k the seven accumulators are drained into two 64-bit integers per output (exact), and
-// the only roundings are the slicing, the dropped weights d >= 7 (2^-56 of |row| |column| per term) and the final
-// conversion: about a quarter of what FP64 FMAs accumulate (2^-53 of the partial sum per term, half that on average).
+// the only roundings are the slicing, the dropped weights d >= 7 (at most 6 x 2^-56 = 8e-17 of max |row| max |column| per
+// term, after the scales; rms about 2^-56) and the final conversion.  The bound is normwise: where a row's large elements
+// meet zeros of a column and its small ones carry that output, FP64 FMAs keep more of it.  On the path's data the error is
+// about a quarter of what they accumulate (2^-53 of the partial sum per term, half that on average; rms below).
 //
 // Why: the FP64 pipe does 2 FMA per clock and SM (0.95 TFLOP/s in this engine's SIMT GEMM); 28 digit products of BF16
-// are 28 / 4096 of a clock per FP64 FMA.  Bound by the MMAs' operand reads from L2: a 128 x 64 tile moves 84 KB per
-// 32 k, 900 tensor clocks per 16.  Measured (FP64 SIMT before -> with slicing): sep1 3366 x 580 x 6384 25.2 -> 1.01 ms,
+// are 28 / 4096 of a clock per FP64 FMA.  A k block of 32 takes 2180 clocks, 1792 of them tensor work, with its 84 KB of
+// operands from L2 underneath; with few k blocks (the xi groups: 17k of a tile's 44k clocks) the drains, the rounding and
+// the set-up take the rest.  Measured (FP64 SIMT before -> with slicing): sep1 3366 x 580 x 6384 25.2 -> 1.01 ms,
 // Hankel 3366 x 796 x 2687 11.0 -> 0.53, kappa 2400 x 798 x 3366 13.8 -> 0.57, sep2 3366 x 2687 x 446 6.8 -> 0.40, the xi
 // groups (67 GFLOP, K about 300) 70.4 -> 5.0 (6.5 with row-wise scattered stores and FP64 conversions in the epilogue); rms error on such data 6e-17 .. 5e-16 against 6e-16 .. 3e-15.
 //

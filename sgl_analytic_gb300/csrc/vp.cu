@@ -24,7 +24,7 @@
 // Phase 2 (k_vp_chain): one thread per point walks the shells: projection, alpha' = K^T alpha (or the
 // stationary weights at s = 0) times exp(z - max Re z), renormalisation by max |alpha|, log scale;
 // FP64, thread-private shared memory, no barriers.  The mixed path's chain (k_vp_chain_ff) is the same recursion in
-// float-float.
+// float-float; points where its range could tell are done over by k_vp_chain.
 #include "kernels.cuh"
 
 namespace sgl {
@@ -747,7 +747,8 @@ __device__ __forceinline__ ff ff_reduce(ff x, float q, float c1, float c2h, floa
     return ff_quick(s.hi, s.lo + ((x.lo - e) - q * c2l));
 }
 
-// e^x, x <= 0: x = n ln 2 + r, 1 + r + r^2 / 2 + r^3 / 6 in float-float, the rest (6e-4 of the value) in FP32; results down
+// e^x, x <= 0: x = n ln 2 + r with ln 2 as a short head and a tail (Cody & Waite, Software Manual for the Elementary
+// Functions, 1980; the same for pi / 2 below), 1 + r + r^2 / 2 + r^3 / 6 in float-float, the rest (6e-4 of the value) in FP32; results down
 // to the subnormal numbers, 0 below 2^-150
 __device__ __forceinline__ ff ff_exp(ff x) {
     ff z = {0.f, 0.f};
