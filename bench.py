@@ -197,10 +197,9 @@ def run_reference(args, rank, world):
     print(json.dumps(line))
 
 
-# FP32-pipe operations per (k, cell) term of the mixed sweep, counted from the kernel source:
-# float-float product 3, half-angle reduction 8, sincosf on the reduced argument ~14,
-# cos-1 / sin-ph / small-argument select 6, two Kahan updates 8.
-MIXED_OPS_PER_TERM = 39
+# FP32-pipe operations per (k, cell) term of the mixed sweep, counted from the kernel source (packed over
+# two cells): phase and reduction 10, the two polynomials with their factors 17, weights 2, Kahan sums 1.5.
+MIXED_OPS_PER_TERM = 31
 
 
 def run_cf_sweep(args, rank, world, local):
